@@ -19,6 +19,7 @@
 #include <cuda_runtime.h>
 
 #include <cmath>
+#include <cstdint>
 #include <cstring>
 #include <string>
 #include <vector>
@@ -42,52 +43,151 @@ constexpr float kClip = 8.0f;  // standardised inputs are clipped to +-kClip (st
 
 // ---------------------------------------------------------------- projection
 struct ProjParams {
-    int nxc, nyc, nzc, f;
+    int nxc, nyc, nzc;
     float P[4][32];  // P[i][a]: coarse node i from fine sample a (a < 4 f)
 };
 
+// x-contracted samples of one coarse element and variable, [b][c] float4 over
+// the coarse i; rows of 4 f + 2 so that the 8 lanes of a 128-bit store phase
+// (4 values of b, 2 of c) hit distinct banks.
+template <int f>
+struct ProjSlot {
+    static constexpr int F = 4 * f, row = F + 2;
+    // coarse elements per block: 16 f^2 threads each (one per fine x-line of
+    // the element's cross-section), so that small factors fill a block too
+    static constexpr int epb = f >= 3 ? 1 : f == 2 ? 4 : 16;
+    float4 t1[5][F * row];
+    float4 t2[5][F * 4];   // y-contracted: [c][j] over i
+};
+
+// VEC: the planes are 16-byte aligned (any caller's pointer is accepted)
+template <bool VEC, class TS>
+__device__ __forceinline__ float4 proj_load4(const TS* p) {
+    if constexpr (!VEC) {
+        return make_float4((float)p[0], (float)p[1], (float)p[2], (float)p[3]);
+    } else if constexpr (sizeof(TS) == 4) {
+        return __ldcs(reinterpret_cast<const float4*>(p));
+    } else {
+        const double2 a = __ldcs(reinterpret_cast<const double2*>(p));
+        const double2 b = __ldcs(reinterpret_cast<const double2*>(p) + 1);
+        return make_float4((float)a.x, (float)a.y, (float)b.x, (float)b.y);
+    }
+}
+
+template <bool VEC, class TD>
+__device__ __forceinline__ void proj_store4(TD* p, const float4& v) {
+    if constexpr (!VEC) {
+        p[0] = (TD)v.x;
+        p[1] = (TD)v.y;
+        p[2] = (TD)v.z;
+        p[3] = (TD)v.w;
+    } else if constexpr (sizeof(TD) == 4) {
+        *reinterpret_cast<float4*>(p) = v;
+    } else {
+        reinterpret_cast<double2*>(p)[0] = make_double2((double)v.x, (double)v.y);
+        reinterpret_cast<double2*>(p)[1] = make_double2((double)v.z, (double)v.w);
+    }
+}
+
+__device__ __forceinline__ void axpy4(float c, const float4& x, float4& y) {
+    y.x += c * x.x;
+    y.y += c * x.y;
+    y.z += c * x.z;
+    y.w += c * x.w;
+}
+
+// Sum-factorised projection, bound by reading the fine state once. A thread
+// owns one (b, c) line of fine samples of its coarse element: 16 consecutive
+// lanes read the 16 x-lines of a fine element (256 contiguous bytes as
+// 128-bit loads) and contract x in registers over the f fine elements of the
+// line, for all five variables (5 f loads in flight). y and z are contracted
+// from shared memory, four coarse i per 128-bit access, one task per
+// (variable, c, j) and (variable, k, j). Every sum runs over its fine samples
+// in ascending order. 96^3 f32 onto 24^3 (1.13 GB read, 170 us at the copy
+// rate) with the features of the result: 1421 us a call when a block gathered
+// one sample a thread per variable, 224 us so.
+template <class TS, class TD, int f, bool VEC>
+__global__ void __launch_bounds__(16 * f * f * ProjSlot<f>::epb)
+    project_kernel(const TS* __restrict__ src, TD* __restrict__ dst, const ProjParams pp) {
+    constexpr int F = 4 * f, T = 16 * f * f, G = ProjSlot<f>::epb;
+    extern __shared__ __align__(16) unsigned char proj_smem[];
+    const int g = threadIdx.x / T, t = threadIdx.x - g * T;
+    ProjSlot<f>& sm = reinterpret_cast<ProjSlot<f>*>(proj_smem)[g];
+    const long long nec = (long long)pp.nxc * pp.nyc * pp.nzc;
+    const long long ec = (long long)blockIdx.x * G + g;
+    const bool live = ec < nec;
+    const long long npc = nec * 64, npf = npc * (f * f * f);
+    {
+        const unsigned e = (unsigned)(live ? ec : 0);
+        const unsigned r = e / (unsigned)pp.nxc, cx = e - r * (unsigned)pp.nxc;
+        const unsigned cz = r / (unsigned)pp.nyc, cy = r - cz * (unsigned)pp.nyc;
+        const int l = t & 15, qy = (t >> 4) % f, qz = (t >> 4) / f;
+        const long long nxf = (long long)pp.nxc * f, nyf = (long long)pp.nyc * f;
+        const long long fe = (long long)cx * f + nxf * ((long long)cy * f + qy + nyf * ((long long)cz * f + qz));
+        const TS* p = src + fe * 64 + 4 * l;
+        const int at = (4 * qy + (l & 3)) * ProjSlot<f>::row + 4 * qz + (l >> 2);
+#pragma unroll(f <= 4 ? 5 : 1)
+        for (int v = 0; v < 5; ++v) {
+            float4 w[f];
+#pragma unroll
+            for (int q = 0; q < f; ++q) w[q] = proj_load4<VEC>(p + v * npf + q * 64);
+            float a[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll
+            for (int q = 0; q < f; ++q)
+#pragma unroll
+                for (int i = 0; i < 4; ++i) {
+                    a[i] += pp.P[i][4 * q + 0] * w[q].x;
+                    a[i] += pp.P[i][4 * q + 1] * w[q].y;
+                    a[i] += pp.P[i][4 * q + 2] * w[q].z;
+                    a[i] += pp.P[i][4 * q + 3] * w[q].w;
+                }
+            sm.t1[v][at] = make_float4(a[0], a[1], a[2], a[3]);
+        }
+    }
+    __syncthreads();
+    for (int s = t; s < 5 * 4 * F; s += T) {
+        const int j = s & 3, c = (s >> 2) % F, v = (s >> 2) / F;
+        float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+        for (int b = 0; b < F; ++b) axpy4(pp.P[j][b], sm.t1[v][b * ProjSlot<f>::row + c], acc);
+        sm.t2[v][c * 4 + j] = acc;
+    }
+    __syncthreads();
+    if (!live) return;
+    for (int s = t; s < 5 * 16; s += T) {
+        const int j = s & 3, k = (s >> 2) & 3, v = s >> 4;
+        float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+        for (int c = 0; c < F; ++c) axpy4(pp.P[k][c], sm.t2[v][c * 4 + j], acc);
+        proj_store4<VEC>(dst + v * npc + ec * 64 + 4 * (s & 15), acc);
+    }
+}
+
+template <class TS, class TD, int f>
+cudaError_t launch_project(const void* src, void* dst, const ProjParams& pp, cudaStream_t s) {
+    constexpr int G = ProjSlot<f>::epb;
+    const size_t sm = sizeof(ProjSlot<f>) * G;
+    const long long ne = (long long)pp.nxc * pp.nyc * pp.nzc;
+    // 128-bit accesses on 16-byte aligned buffers (what cudaMalloc and torch give), scalar ones on others
+    const bool vec = ((reinterpret_cast<uintptr_t>(src) | reinterpret_cast<uintptr_t>(dst)) & 15) == 0;
+    auto* fn = vec ? project_kernel<TS, TD, f, true> : project_kernel<TS, TD, f, false>;
+    cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
+    if (e != cudaSuccess) return e;
+    fn<<<(unsigned)((ne + G - 1) / G), 16 * f * f * G, sm, s>>>((const TS*)src, (TD*)dst, pp);
+    return cudaGetLastError();
+}
+
 template <class TS, class TD>
-__global__ void __launch_bounds__(256) project_kernel(const TS* __restrict__ src, TD* __restrict__ dst,
-                                                      ProjParams pp) {
-    extern __shared__ float sh[];  // (4f)^3 fine samples, then 4 x (4f)^2, then 16 x 4f
-    const int F = 4 * pp.f;
-    float* u = sh;
-    float* t1 = u + F * F * F;
-    float* t2 = t1 + 4 * F * F;
-    const long long ec = blockIdx.x;
-    const int cx = (int)(ec % pp.nxc), cy = (int)((ec / pp.nxc) % pp.nyc), cz = (int)(ec / ((long long)pp.nxc * pp.nyc));
-    const long long nxf = (long long)pp.nxc * pp.f, nyf = (long long)pp.nyc * pp.f, nzf = (long long)pp.nzc * pp.f;
-    const long long npf = nxf * nyf * nzf * 64, npc = (long long)pp.nxc * pp.nyc * pp.nzc * 64;
-    for (int v = 0; v < 5; ++v) {
-        __syncthreads();
-        for (int s = threadIdx.x; s < F * F * F; s += blockDim.x) {
-            const int a = s % F, b = (s / F) % F, c = s / (F * F);
-            const long long fe = (cx * pp.f + a / 4) + nxf * ((cy * pp.f + b / 4) + nyf * (long long)(cz * pp.f + c / 4));
-            u[s] = (float)src[v * npf + fe * 64 + (a & 3) + 4 * (b & 3) + 16 * (c & 3)];
-        }
-        __syncthreads();
-        // x: t1[i][b][c]
-        for (int s = threadIdx.x; s < 4 * F * F; s += blockDim.x) {
-            const int i = s & 3, bc = s >> 2;
-            float acc = 0.f;
-            for (int a = 0; a < F; ++a) acc += pp.P[i][a] * u[a + F * bc];
-            t1[s] = acc;  // index i + 4 (b + F c)
-        }
-        __syncthreads();
-        // y: t2[i][j][c]
-        for (int s = threadIdx.x; s < 16 * F; s += blockDim.x) {
-            const int i = s & 3, j = (s >> 2) & 3, c = s >> 4;
-            float acc = 0.f;
-            for (int b = 0; b < F; ++b) acc += pp.P[j][b] * t1[i + 4 * (b + F * c)];
-            t2[s] = acc;  // index i + 4 j + 16 c
-        }
-        __syncthreads();
-        if (threadIdx.x < 64) {
-            const int i = threadIdx.x & 3, j = (threadIdx.x >> 2) & 3, k = threadIdx.x >> 4;
-            float acc = 0.f;
-            for (int c = 0; c < F; ++c) acc += pp.P[k][c] * t2[i + 4 * j + 16 * c];
-            dst[v * npc + ec * 64 + threadIdx.x] = (TD)acc;
-        }
+cudaError_t launch_project_f(int f, const void* src, void* dst, const ProjParams& pp, cudaStream_t s) {
+    switch (f) {
+        case 1: return launch_project<TS, TD, 1>(src, dst, pp, s);
+        case 2: return launch_project<TS, TD, 2>(src, dst, pp, s);
+        case 3: return launch_project<TS, TD, 3>(src, dst, pp, s);
+        case 4: return launch_project<TS, TD, 4>(src, dst, pp, s);
+        case 5: return launch_project<TS, TD, 5>(src, dst, pp, s);
+        case 6: return launch_project<TS, TD, 6>(src, dst, pp, s);
+        case 7: return launch_project<TS, TD, 7>(src, dst, pp, s);
+        default: return launch_project<TS, TD, 8>(src, dst, pp, s);
     }
 }
 
@@ -96,7 +196,6 @@ ProjParams proj_params(int nxc, int nyc, int nzc, int f) {
     pp.nxc = nxc;
     pp.nyc = nyc;
     pp.nzc = nzc;
-    pp.f = f;
     const od::TablesD t = od::host_fr_tables();
     double w[4];
     for (int a = 0; a < 4; ++a) {
@@ -722,27 +821,14 @@ int od_project(const void* src, int src_f64, int nxc, int nyc, int nzc, int fact
                void* stream) {
     if (!src || !dst || nxc <= 0 || nyc <= 0 || nzc <= 0 || factor < 1 || factor > 8) return OD_ERR_ARG;
     const ProjParams pp = proj_params(nxc, nyc, nzc, factor);
-    const int F = 4 * factor;
-    const size_t sm = sizeof(float) * ((size_t)F * F * F + 4 * F * F + 16 * F);
-    const long long ne = (long long)nxc * nyc * nzc;
     cudaStream_t s = (cudaStream_t)stream;
-    cudaError_t e = cudaSuccess;
-#define OD_PROJ(TS, TD)                                                                                   \
-    do {                                                                                                  \
-        e = cudaFuncSetAttribute(project_kernel<TS, TD>, cudaFuncAttributeMaxDynamicSharedMemorySize,     \
-                                 (int)sm);                                                                \
-        if (e == cudaSuccess) project_kernel<TS, TD><<<(unsigned)ne, 256, sm, s>>>((const TS*)src, (TD*)dst, pp); \
-    } while (0)
-    if (src_f64 && dst_f64)
-        OD_PROJ(double, double);
-    else if (src_f64)
-        OD_PROJ(double, float);
-    else if (dst_f64)
-        OD_PROJ(float, double);
+    cudaError_t e;
+    if (src_f64)
+        e = dst_f64 ? launch_project_f<double, double>(factor, src, dst, pp, s)
+                    : launch_project_f<double, float>(factor, src, dst, pp, s);
     else
-        OD_PROJ(float, float);
-#undef OD_PROJ
-    if (e == cudaSuccess) e = cudaGetLastError();
+        e = dst_f64 ? launch_project_f<float, double>(factor, src, dst, pp, s)
+                    : launch_project_f<float, float>(factor, src, dst, pp, s);
     return e == cudaSuccess ? OD_OK : OD_ERR_CUDA;
 }
 
