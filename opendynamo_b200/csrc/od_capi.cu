@@ -159,6 +159,7 @@ struct od_ctx {
     int slab_z0 = 0, slab_z1 = 0, mesh_nz = 0;   // owned z-layers [z0, z1) of a mesh of mesh_nz layers
     cudaEvent_t ev_halo[2] = {nullptr, nullptr};   // od_slabs_step: stage input ready / face records ready
     size_t buf_bytes = 0;     // one state buffer (state_bytes: the owned part the caller sees)
+    double* diag = nullptr;   // od_diagnostics' sums, allocated by the first call and kept
     // od_get_state_async: device snapshot of the state and its two events
     void* snap = nullptr;
     cudaEvent_t ev_snap = nullptr, ev_copied = nullptr;
@@ -504,6 +505,7 @@ void od_destroy(od_ctx* c) {
         if (c->U[b]) cudaFree(c->U[b]);
     if (c->fv) cudaFree(c->fv);
     if (c->rhs) cudaFree(c->rhs);
+    if (c->diag) cudaFree(c->diag);
     // copies still running on the caller's streams
     if (c->ev_copied) cudaEventSynchronize(c->ev_copied);
     if (c->ev_staged) cudaEventSynchronize(c->ev_staged);
@@ -881,16 +883,22 @@ int od_diagnostics(od_ctx* c, double* vol6, double* prof, size_t prof_len) {
     const size_t nprof = (size_t)c->p.ny * 4 * 8;
     if (prof && prof_len < nprof) return fail(c, OD_ERR_SIZE, "profile buffer smaller than ny*4*8");
     if (int rc = set_device(c)) return rc;
-    double* d = nullptr;
     const size_t bytes = (6 + nprof) * sizeof(double);
-    cudaError_t e = cudaMallocAsync((void**)&d, bytes, c->stream);
-    if (e == cudaSuccess) e = cudaMemsetAsync(d, 0, bytes, c->stream);
+    cudaError_t e = cudaSuccess;
+    // kept by the context: an allocation from the pool and its release on
+    // every call cost several times the kernel's own time
+    double* d = c->diag;
+    if (!d) {
+        e = cudaMalloc((void**)&d, bytes);
+        if (e != cudaSuccess) return cuda_fail(c, e, "diagnostics workspace");
+        c->diag = d;
+    }
+    e = cudaMemsetAsync(d, 0, bytes, c->stream);
     if (e == cudaSuccess)
         e = od::launch_diag(c->U[0], c->elem_size == 8, c->p.nx, c->p.ny, c->p.nz, c->p.lx, c->p.ly, c->p.lz,
                             c->tab, d, prof ? d + 6 : nullptr, c->stream);
     std::vector<double> h(6 + nprof);
     if (e == cudaSuccess) e = cudaMemcpyAsync(h.data(), d, bytes, cudaMemcpyDeviceToHost, c->stream);
-    if (d) cudaFreeAsync(d, c->stream);
     if (e == cudaSuccess) e = cudaStreamSynchronize(c->stream);
     if (e != cudaSuccess) return cuda_fail(c, e, "diagnostics");
     std::copy(h.begin(), h.begin() + 6, vol6);
