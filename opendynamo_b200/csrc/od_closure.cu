@@ -32,6 +32,7 @@ namespace od {
 TablesD host_fr_tables();
 namespace mlp {
 cudaError_t launch_gemm(const GemmArgs& g, int epi, cudaStream_t s, size_t ws_floats);
+cudaError_t launch_gemm_group(GemmArgs* g, int n, float* ws, size_t ws_floats, cudaStream_t s);
 }
 }  // namespace od
 
@@ -387,82 +388,282 @@ __global__ void apply_kernel(T* __restrict__ rhs, const float* __restrict__ Y, l
 }
 
 // ---------------------------------------------------------------- training kernels
+// The operands of the weight-gradient products are wanted twice, row-major
+// and transposed. Every kernel here that writes both goes through a tile of
+// 64 columns in shared memory and writes 16-byte chunks in both orientations
+// (a 2-byte store per value into the transposed copy touched a sector each:
+// at a batch of 8192 the gather took 80 us and the loss gradient 129 us, both
+// about 8 us of traffic).
+
+// shared-memory position of (row r, column c) of a tile of 64 columns: the
+// row's 16-byte chunks are XORed with its row group, so that whole-row writes
+// and reads of eight row groups of one column both hit distinct banks
+__device__ __forceinline__ int tr_at(int r, int c) { return r * 64 + (c ^ (((r >> 3) & 7) << 3)); }
+
+__device__ __forceinline__ uint4 pack8(const bf16* v) {
+    uint4 o;
+    o.x = (uint32_t)__bfloat16_as_ushort(v[0]) | ((uint32_t)__bfloat16_as_ushort(v[1]) << 16);
+    o.y = (uint32_t)__bfloat16_as_ushort(v[2]) | ((uint32_t)__bfloat16_as_ushort(v[3]) << 16);
+    o.z = (uint32_t)__bfloat16_as_ushort(v[4]) | ((uint32_t)__bfloat16_as_ushort(v[5]) << 16);
+    o.w = (uint32_t)__bfloat16_as_ushort(v[6]) | ((uint32_t)__bfloat16_as_ushort(v[7]) << 16);
+    return o;
+}
+
+// rows 8 rc .. 8 rc + 7 of column c of the tile
+__device__ __forceinline__ uint4 tr_column(const bf16* tile, int rc, int c) {
+    bf16 v[8];
+#pragma unroll
+    for (int i = 0; i < 8; ++i) v[i] = tile[tr_at(8 * rc + i, c)];
+    return pack8(v);
+}
+
+// eight values of a caller's pool; VEC: the pool is 16-byte aligned
+template <bool VEC>
+__device__ __forceinline__ uint4 pool8(const bf16* p) {
+    if constexpr (VEC) {
+        return __ldg(reinterpret_cast<const uint4*>(p));
+    } else {
+        bf16 v[8];
+#pragma unroll
+        for (int i = 0; i < 8; ++i) v[i] = p[i];
+        return pack8(v);
+    }
+}
+
+// rows of the bf16 feature pool into a batch: X [M x 896] and X^T; rows past
+// mv are zero. Block (x, y): 64 rows, 64 columns.
+template <bool VEC>
+__global__ void __launch_bounds__(256) gather_kernel(const bf16* __restrict__ Xp, const long long* __restrict__ rows,
+                                                     int mv, int M, bf16* __restrict__ X, bf16* __restrict__ XT) {
+    __shared__ __align__(16) bf16 tile[64 * 64];
+    const int m0 = blockIdx.x * 64, c0 = blockIdx.y * 64;
+#pragma unroll
+    for (int q = 0; q < 2; ++q) {
+        const int r = (threadIdx.x + 256 * q) >> 3, c = (threadIdx.x & 7) * 8, m = m0 + r;
+        uint4 v = make_uint4(0, 0, 0, 0);
+        if (m < mv) v = pool8<VEC>(Xp + rows[m] * kIn + c0 + c);
+        *reinterpret_cast<uint4*>(X + (size_t)m * kIn + c0 + c) = v;
+        *reinterpret_cast<uint4*>(&tile[tr_at(r, c)]) = v;
+    }
+    __syncthreads();
+#pragma unroll
+    for (int q = 0; q < 2; ++q) {
+        const int c = (threadIdx.x + 256 * q) >> 3, rc = threadIdx.x & 7;
+        *reinterpret_cast<uint4*>(XT + (size_t)(c0 + c) * M + m0 + 8 * rc) = tr_column(tile, rc, c);
+    }
+}
+
 // dY = g (Y - T) on the valid block (rows < mv, columns < kOut), 0 elsewhere;
-// bf16 [M x 384] and its transpose; loss += sum (Y - T)^2
-__global__ void loss_grad_kernel(const float* __restrict__ Y, const float* __restrict__ T, int M, int mv, float g,
-                                 bf16* __restrict__ dY, bf16* __restrict__ dYT, double* loss) {
-    const long long idx = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    float sq = 0.f;
-    if (idx < (long long)M * kOutPad) {
-        const int m = (int)(idx / kOutPad), n = (int)(idx % kOutPad);
-        float d = 0.f;
-        if (m < mv && n < kOut) {
-            const float r = Y[idx] - T[idx];
-            d = g * r;
-            sq = r * r;
+// bf16 [M x 384] and its transpose; loss += sum (Y - T)^2. The targets are
+// fp32 rows [M x 384], or (POOL) rows of the bf16 target pool [n x 320].
+// Block (x, y): 64 rows, 64 columns.
+template <bool POOL, bool VEC>
+__global__ void __launch_bounds__(256) loss_grad_kernel(const float* __restrict__ Y, const float* __restrict__ T,
+                                                        const bf16* __restrict__ Tp, const long long* __restrict__ rows,
+                                                        int M, int mv, float g, bf16* __restrict__ dY,
+                                                        bf16* __restrict__ dYT, double* loss) {
+    __shared__ __align__(16) bf16 tile[64 * 64];
+    __shared__ double red[8];
+    const int m0 = blockIdx.x * 64, n0 = blockIdx.y * 64;
+    double sq = 0.0;
+#pragma unroll
+    for (int q = 0; q < 2; ++q) {
+        const int r = (threadIdx.x + 256 * q) >> 3, c = (threadIdx.x & 7) * 8, m = m0 + r;
+        uint4 o = make_uint4(0, 0, 0, 0);
+        if (m < mv && n0 < kOut) {   // kOut is a multiple of 64
+            const size_t at = (size_t)m * kOutPad + n0 + c;
+            float y[8], t[8];
+#pragma unroll
+            for (int h = 0; h < 2; ++h)
+                *reinterpret_cast<float4*>(y + 4 * h) = __ldg(reinterpret_cast<const float4*>(Y + at) + h);
+            if constexpr (POOL) {
+                const uint4 w = pool8<VEC>(Tp + rows[m] * kOut + n0 + c);
+                const uint32_t u[4] = {w.x, w.y, w.z, w.w};
+#pragma unroll
+                for (int i = 0; i < 4; ++i) {
+                    t[2 * i] = __uint_as_float(u[i] << 16);
+                    t[2 * i + 1] = __uint_as_float(u[i] & 0xffff0000u);
+                }
+            } else {
+#pragma unroll
+                for (int h = 0; h < 2; ++h)
+                    *reinterpret_cast<float4*>(t + 4 * h) = __ldg(reinterpret_cast<const float4*>(T + at) + h);
+            }
+            bf16 b[8];
+#pragma unroll
+            for (int i = 0; i < 8; ++i) {
+                const float d = y[i] - t[i];
+                b[i] = __float2bfloat16_rn(g * d);
+                sq += (double)(d * d);
+            }
+            o = pack8(b);
         }
-        const bf16 b = __float2bfloat16_rn(d);
-        dY[idx] = b;
-        dYT[(long long)n * M + m] = b;
+        *reinterpret_cast<uint4*>(dY + (size_t)m * kOutPad + n0 + c) = o;
+        *reinterpret_cast<uint4*>(&tile[tr_at(r, c)]) = o;
     }
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) sq += __shfl_down_sync(0xffffffffu, sq, o);
-    if ((threadIdx.x & 31) == 0 && sq != 0.f) atomicAdd(loss, (double)sq);
-}
-
-// out[n] = sum_m AT[n][m] (bf16 -> fp32): bias gradients from the transposed
-// copies, one block per row, coalesced
-__global__ void __launch_bounds__(256) rowsum_kernel(const bf16* __restrict__ AT, int M, float* __restrict__ out) {
-    __shared__ float red[8];
-    const bf16* row = AT + (long long)blockIdx.x * M;
-    float s = 0.f;
-    for (int m = threadIdx.x; m < M; m += blockDim.x) s += __bfloat162float(row[m]);
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) s += __shfl_down_sync(0xffffffffu, s, o);
-    if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = s;
+    if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = sq;
     __syncthreads();
-    if (threadIdx.x == 0) {
-        float t = 0.f;
-        for (int w = 0; w < 8; ++w) t += red[w];
-        out[blockIdx.x] = t;
+#pragma unroll
+    for (int q = 0; q < 2; ++q) {
+        const int c = (threadIdx.x + 256 * q) >> 3, rc = threadIdx.x & 7;
+        *reinterpret_cast<uint4*>(dYT + (size_t)(n0 + c) * M + m0 + 8 * rc) = tr_column(tile, rc, c);
+    }
+    if (threadIdx.x == 0 && n0 < kOut) {
+        double s = 0.0;
+#pragma unroll
+        for (int w = 0; w < 8; ++w) s += red[w];
+        atomicAdd(loss, s);
     }
 }
 
-// rows of a bf16 pool (and a bf16 target pool) into a batch: X [M x 896], X^T, T [M x 384] fp32
-__global__ void gather_kernel(const bf16* __restrict__ Xp, const bf16* __restrict__ Tp, const long long* __restrict__ rows,
-                              int mv, int M, bf16* __restrict__ X, bf16* __restrict__ XT, float* __restrict__ T) {
-    const long long idx = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (idx < (long long)M * kIn) {
-        const int m = (int)(idx / kIn), c = (int)(idx % kIn);
-        const bf16 v = m < mv ? Xp[rows[m] * kIn + c] : __float2bfloat16_rn(0.f);
-        X[idx] = v;
-        XT[(long long)c * M + m] = v;
+// The end of the backward pass in one launch: bias gradients out[n] = sum_m
+// AT[n][m] (bf16 -> fp32) from the transposed copies, and the sums of the
+// weight gradients' K ranges. Launched one by one they took 35 and 27 us at a
+// batch of 8192, each waiting for its first loads alone; together 19 us.
+//
+// Row sums, a warp per row: the order is that of 256 partial sums s[t] =
+// AT[n][t] + AT[n][t + 256] + ..., each 32 of them summed in a tree (t + 16,
+// t + 8, ... + 1), the eight trees in sequence: Adam's first steps divide by
+// the gradient's own size, so another order moves the weights. Lane l holds
+// the partial sums 8 l .. 8 l + 7 and loads 16 bytes at a time (M % 8 == 0).
+// K ranges: one value a thread, in ascending order, 16 loads in flight.
+constexpr int kFinishThreads = 128;
+
+struct GradFinish {
+    const bf16* AT[4];      // [rows x M]
+    float* bias[4];
+    const float* ws[4];     // [ks x mn]
+    float* w[4];
+    long long mn[4];
+    int ks[4];
+    int first_b[5], first_w[5];   // blocks of each row-sum part, then of each K-range part
+    int M;
+};
+
+__device__ __forceinline__ float row_sum(const bf16* AT, int M, int n, int lane) {
+    const uint4* row = reinterpret_cast<const uint4*>(AT + (size_t)n * M);
+    float s[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+#pragma unroll 8
+    for (int q = lane; q < M / 8; q += 32) {
+        const uint4 w = __ldg(row + q);
+        const uint32_t u[4] = {w.x, w.y, w.z, w.w};
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            s[2 * i] += __uint_as_float(u[i] << 16);
+            s[2 * i + 1] += __uint_as_float(u[i] & 0xffff0000u);
+        }
     }
-    if (idx < (long long)M * kOutPad) {
-        const int m = (int)(idx / kOutPad), c = (int)(idx % kOutPad);
-        T[idx] = (m < mv && c < kOut) ? __bfloat162float(Tp[rows[m] * kOut + c]) : 0.f;
-    }
+#pragma unroll
+    for (int o = 2; o > 0; o >>= 1)
+#pragma unroll
+        for (int i = 0; i < 8; ++i) s[i] += __shfl_down_sync(0xffffffffu, s[i], o, 4);
+#pragma unroll
+    for (int o = 4; o > 0; o >>= 1)
+#pragma unroll
+        for (int i = 0; i < o; ++i) s[i] += s[i + o];
+    float t = 0.f;
+#pragma unroll
+    for (int w = 0; w < 8; ++w) t += __shfl_sync(0xffffffffu, s[0], 4 * w);
+    return t;
 }
 
-// Adam on fp32 master weights, then the bf16 copies (W and W^T) of the layer
-__global__ void adam_kernel(float* __restrict__ w, const float* __restrict__ g, float* __restrict__ m1,
-                            float* __restrict__ m2, long long n, float lr, float b1, float b2, float eps, float c1,
-                            float c2, int rows, int cols, bf16* __restrict__ wb, bf16* __restrict__ wbT) {
-    const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    const float gi = g[i];
-    const float a = b1 * m1[i] + (1.f - b1) * gi;
-    const float b = b2 * m2[i] + (1.f - b2) * gi * gi;
-    m1[i] = a;
-    m2[i] = b;
-    const float wn = w[i] - lr * (a / c1) / (sqrtf(b / c2) + eps);
-    w[i] = wn;
-    if (wb) {
-        const bf16 h = __float2bfloat16_rn(wn);
-        wb[i] = h;
-        const int r = (int)(i / cols), c = (int)(i % cols);
-        wbT[(long long)c * rows + r] = h;
+__global__ void __launch_bounds__(kFinishThreads) grad_finish_kernel(const GradFinish F) {
+    const int b = (int)blockIdx.x;
+    if (b < F.first_b[4]) {
+        int l = 0;
+        while (b >= F.first_b[l + 1]) ++l;
+        const int n = (b - F.first_b[l]) * (kFinishThreads / 32) + (threadIdx.x >> 5), lane = threadIdx.x & 31;
+        const float t = row_sum(F.AT[l], F.M, n, lane);
+        if (lane == 0) F.bias[l][n] = t;
+        return;
     }
+    int l = 0;
+    while (b >= F.first_w[l + 1]) ++l;
+    const long long i = (long long)(b - F.first_w[l]) * kFinishThreads + threadIdx.x, mn = F.mn[l];
+    const float* p = F.ws[l] + i;
+    const int ks = F.ks[l];
+    float v = 0.f;
+#pragma unroll 16
+    for (int z = 0; z < ks; ++z) v += __ldcs(p + z * mn);
+    F.w[l][i] = v;
+}
+
+struct AdamStep {
+    float lr, b1, b2, eps, c1, c2;
+};
+
+// The two moments' multiply-adds are pinned: where the compiler contracts them
+// depends on the code around, and an early step, which divides by the
+// gradient's own size, carries the last bit of them into the weights.
+__device__ __forceinline__ float adam_update(const AdamStep& p, float w, float g, float& m1, float& m2) {
+    const float a = __fmaf_rn(1.f - p.b1, g, __fmul_rn(p.b1, m1));
+    const float b = __fmaf_rn(__fmul_rn(1.f - p.b2, g), g, __fmul_rn(p.b2, m2));
+    m1 = a;
+    m2 = b;
+    return w - p.lr * (a / p.c1) / (sqrtf(b / p.c2) + p.eps);
+}
+
+// the flat parameter layout of all layers and the bf16 copies made from it
+struct AdamArgs {
+    float *w, *m1, *m2;
+    const float* g;
+    long long off_w[4], off_b[4];
+    int rows[4], cols[4];
+    bf16 *wb[4], *wbT[4];
+    bf16* wt;
+    AdamStep p;
+};
+
+constexpr int kAdamRows = 32;   // rows of a weight tile (of 64 columns)
+
+// Adam on the fp32 master weights of every layer in one launch: blocks 0..:
+// weight tiles of 32 rows x 64 columns, which also write the bf16 copies W and
+// W^T and the fused inference kernel's weight image; the last four blocks: the
+// layers' biases. (Eight launches of one value a thread with 2-byte stores
+// into W^T, and a ninth for the image, took 39 us; this one 9 us.)
+__global__ void __launch_bounds__(256) adam_kernel(const AdamArgs A, int tiles) {
+    __shared__ __align__(16) bf16 tile[kAdamRows * 64];
+    int b = blockIdx.x, l = 0;
+    if (b >= tiles) {
+        l = b - tiles;
+        const long long o = A.off_b[l];
+        for (int i = threadIdx.x; i < A.rows[l]; i += 256)
+            A.w[o + i] = adam_update(A.p, A.w[o + i], A.g[o + i], A.m1[o + i], A.m2[o + i]);
+        return;
+    }
+    for (int n; b >= (n = (A.rows[l] / kAdamRows) * (A.cols[l] / 64)); ++l) b -= n;
+    const int cb = A.cols[l] / 64, kb = b % cb, r0 = b / cb * kAdamRows, cols = A.cols[l], rows = A.rows[l];
+    const int r = threadIdx.x >> 3, kc = threadIdx.x & 7;
+    const long long at = A.off_w[l] + (long long)(r0 + r) * cols + kb * 64 + 8 * kc;
+    bf16 h[8];
+#pragma unroll
+    for (int q = 0; q < 2; ++q) {
+        float4 w = *reinterpret_cast<const float4*>(A.w + at + 4 * q);
+        float4 m1 = *reinterpret_cast<const float4*>(A.m1 + at + 4 * q);
+        float4 m2 = *reinterpret_cast<const float4*>(A.m2 + at + 4 * q);
+        const float4 g = *reinterpret_cast<const float4*>(A.g + at + 4 * q);
+        w.x = adam_update(A.p, w.x, g.x, m1.x, m2.x);
+        w.y = adam_update(A.p, w.y, g.y, m1.y, m2.y);
+        w.z = adam_update(A.p, w.z, g.z, m1.z, m2.z);
+        w.w = adam_update(A.p, w.w, g.w, m1.w, m2.w);
+        *reinterpret_cast<float4*>(A.w + at + 4 * q) = w;
+        *reinterpret_cast<float4*>(A.m1 + at + 4 * q) = m1;
+        *reinterpret_cast<float4*>(A.m2 + at + 4 * q) = m2;
+        h[4 * q] = __float2bfloat16_rn(w.x);
+        h[4 * q + 1] = __float2bfloat16_rn(w.y);
+        h[4 * q + 2] = __float2bfloat16_rn(w.z);
+        h[4 * q + 3] = __float2bfloat16_rn(w.w);
+    }
+    const uint4 o = pack8(h);
+    *reinterpret_cast<uint4*>(A.wb[l] + (size_t)(r0 + r) * cols + kb * 64 + 8 * kc) = o;
+    const uint32_t img = od::mlp::fused_image_off(l, r0 + r, kb, kc);
+    if (img < od::mlp::kFusedWeightBytes) *reinterpret_cast<uint4*>(reinterpret_cast<char*>(A.wt) + img) = o;
+    *reinterpret_cast<uint4*>(&tile[tr_at(r, 8 * kc)]) = o;
+    __syncthreads();
+    const int c = threadIdx.x >> 2, rc = threadIdx.x & 3;
+    *reinterpret_cast<uint4*>(A.wbT[l] + (size_t)(kb * 64 + c) * rows + r0 + 8 * rc) = tr_column(tile, rc, c);
 }
 
 // bf16 copies of all layers from the fp32 master weights
@@ -480,6 +681,8 @@ __global__ void f32_to_bf16_kernel(const float* __restrict__ a, bf16* __restrict
     const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     if (i < n) b[i] = __float2bfloat16_rn(a[i]);
 }
+
+bool aligned16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15) == 0; }
 
 unsigned blocks(long long n, int t) { return (unsigned)((n + t - 1) / t); }
 
@@ -502,12 +705,12 @@ struct od_mlp {
     bf16 *A[3] = {}, *AT[3] = {};
     float* Y = nullptr;
     bf16 *dY = nullptr, *dYT = nullptr;
-    bf16 *dZa = nullptr, *dZaT = nullptr, *dZb = nullptr, *dZbT = nullptr;
+    bf16 *dZ[2] = {}, *dZT[3] = {};   // row-major: a layer and the one above; transposed: kept for the weight gradients
     bf16 *X = nullptr, *XT = nullptr;   // gathered batch (training)
     float* T = nullptr;
     long long* rows_d = nullptr;
-    double* loss = nullptr;
-    int* err = nullptr;
+    double* loss = nullptr;         // 16 bytes: the loss sum, then err
+    int* err = nullptr;             // set by a timed-out wait
     float* ws = nullptr;            // split-K partial sums of the weight gradients
     size_t ws_floats = 0;
     long long step = 0;
@@ -572,44 +775,72 @@ cudaError_t forward(od_mlp* m, const bf16* X, int M, float* Y, bool keep_t) {
 }
 
 // gradients of 1/(mv*320) sum (Y - T)^2 w.r.t. all parameters into m->g
-cudaError_t backward(od_mlp* m, const bf16* XT, int M, int mv) {
-    cudaError_t e = cudaMemsetAsync(m->loss, 0, sizeof(double), m->stream);
+// (targets: m->T, or the gathered rows of the pool Tp)
+cudaError_t backward(od_mlp* m, const bf16* XT, int M, int mv, const bf16* Tp) {
+    cudaError_t e = cudaSuccess;
     const float gs = 2.0f / ((float)mv * (float)kOut);
-    loss_grad_kernel<<<blocks((long long)M * kOutPad, 256), 256, 0, m->stream>>>(m->Y, m->T, M, mv, gs, m->dY,
-                                                                                    m->dYT, m->loss);
+    auto* lg = !Tp ? loss_grad_kernel<false, true>
+                   : aligned16(Tp) ? loss_grad_kernel<true, true> : loss_grad_kernel<true, false>;
+    lg<<<dim3(M / 64, kOutPad / 64), 256, 0, m->stream>>>(m->Y, m->T, Tp, m->rows_d, M, mv, gs, m->dY, m->dYT,
+                                                          m->loss);
     if (e == cudaSuccess) e = cudaGetLastError();
-    // layer 4
-    if (e == cudaSuccess)
-        e = gemm(m, m->dYT, m->AT[2], kOutPad, kHid, M, od::mlp::kStoreF32, nullptr, m->g + m->off_w[3], nullptr,
-                 nullptr, nullptr);
-    rowsum_kernel<<<kOutPad, 256, 0, m->stream>>>(m->dYT, M, m->g + m->off_b[3]);
-    if (e == cudaSuccess)
-        e = gemm(m, m->dY, m->wbT[3], M, kHid, kOutPad, od::mlp::kGeluGrad, nullptr, nullptr, m->dZa, m->dZaT,
-                 m->Z[2]);
-    bf16 *dz = m->dZa, *dzT = m->dZaT, *nz = m->dZb, *nzT = m->dZbT;
+    // down the layers: dZ of the hidden layers, each with its transposed copy
+    const bf16* dz = m->dY;
     for (int l = 2; l >= 0 && e == cudaSuccess; --l) {
-        // weights of layer l: input is A[l-1] (or X for l = 0)
-        const bf16* inT = l == 0 ? XT : m->AT[l - 1];
-        const int kin = l == 0 ? kIn : kHid;
-        e = gemm(m, dzT, inT, kHid, kin, M, od::mlp::kStoreF32, nullptr, m->g + m->off_w[l], nullptr, nullptr,
-                 nullptr);
-        rowsum_kernel<<<kHid, 256, 0, m->stream>>>(dzT, M, m->g + m->off_b[l]);
-        if (e == cudaSuccess && l > 0) {
-            e = gemm(m, dz, m->wbT[l], M, kHid, kHid, od::mlp::kGeluGrad, nullptr, nullptr, nz, nzT, m->Z[l - 1]);
-            std::swap(dz, nz);
-            std::swap(dzT, nzT);
-        }
+        e = gemm(m, dz, m->wbT[l + 1], M, kHid, l == 2 ? kOutPad : kHid, od::mlp::kGeluGrad, nullptr, nullptr,
+                 m->dZ[l & 1], m->dZT[l], m->Z[l]);
+        dz = m->dZ[l & 1];
     }
-    if (e == cudaSuccess) e = cudaGetLastError();
-    return e;
+    // every weight gradient in one launch, then the sums over K ranges and rows
+    od::mlp::GemmArgs g[4] = {};
+    GradFinish F{};
+    F.M = M;
+    int nb = 0;
+    for (int l = 0; l < 4; ++l) {
+        g[l].A = l == 3 ? m->dYT : m->dZT[l];
+        g[l].B = l == 0 ? XT : m->AT[l - 1];
+        g[l].M = m->rows[l];
+        g[l].N = m->cols[l];
+        g[l].K = M;
+        g[l].out_f32 = m->g + m->off_w[l];
+        g[l].err = m->err;
+        F.AT[l] = g[l].A;
+        F.bias[l] = m->g + m->off_b[l];
+        F.first_b[l] = nb;
+        nb += m->rows[l] / (kFinishThreads / 32);
+    }
+    F.first_b[4] = nb;
+    if (e == cudaSuccess) e = od::mlp::launch_gemm_group(g, 4, m->ws, m->ws_floats, m->stream);
+    if (e != cudaSuccess) return e;
+    for (int l = 0; l < 4; ++l) {
+        F.ws[l] = g[l].ws;
+        F.w[l] = g[l].out_f32;
+        F.ks[l] = g[l].ksplit;
+        F.mn[l] = (long long)g[l].M * g[l].N;
+        F.first_w[l] = nb;
+        if (g[l].ksplit > 1) nb += (int)(F.mn[l] / kFinishThreads);
+    }
+    F.first_w[4] = nb;
+    grad_finish_kernel<<<(unsigned)nb, kFinishThreads, 0, m->stream>>>(F);
+    return cudaGetLastError();
 }
 
-int check_err(od_mlp* m) {
-    int h = 0;
-    cudaError_t e = cudaMemcpyAsync(&h, m->err, sizeof(int), cudaMemcpyDeviceToHost, m->stream);
+constexpr size_t kStatusBytes = 16;   // loss and err, cleared and read back together
+
+cudaError_t clear_status(od_mlp* m) { return cudaMemsetAsync(m->loss, 0, kStatusBytes, m->stream); }
+
+// waits for the stream; the loss sum of the calls since clear_status
+int read_status(od_mlp* m, double* loss) {
+    struct {
+        double loss;
+        int err, pad;
+    } h{};
+    static_assert(sizeof h == kStatusBytes, "one copy");
+    cudaError_t e = cudaMemcpyAsync(&h, m->loss, sizeof h, cudaMemcpyDeviceToHost, m->stream);
     if (e == cudaSuccess) e = cudaStreamSynchronize(m->stream);
     if (e != cudaSuccess) return mfail(m, OD_ERR_CUDA, cudaGetErrorString(e));
-    if (h) return mfail(m, OD_ERR_CUDA, "tensor-core GEMM wait timed out");
+    if (loss) *loss = h.loss;
+    if (h.err) return mfail(m, OD_ERR_CUDA, "tensor-core GEMM wait timed out");
     return OD_OK;
 }
 
@@ -665,17 +896,21 @@ int od_mlp_create(int max_rows, int device, od_mlp** out) {
     mal((void**)&m->Y, sizeof(float) * M * kOutPad);
     mal((void**)&m->dY, sizeof(bf16) * M * kOutPad);
     mal((void**)&m->dYT, sizeof(bf16) * M * kOutPad);
-    mal((void**)&m->dZa, sizeof(bf16) * M * kHid);
-    mal((void**)&m->dZaT, sizeof(bf16) * M * kHid);
-    mal((void**)&m->dZb, sizeof(bf16) * M * kHid);
-    mal((void**)&m->dZbT, sizeof(bf16) * M * kHid);
+    for (int l = 0; l < 2; ++l) mal((void**)&m->dZ[l], sizeof(bf16) * M * kHid);
+    for (int l = 0; l < 3; ++l) mal((void**)&m->dZT[l], sizeof(bf16) * M * kHid);
     mal((void**)&m->X, sizeof(bf16) * M * kIn);
     mal((void**)&m->XT, sizeof(bf16) * M * kIn);
     mal((void**)&m->T, sizeof(float) * M * kOutPad);
     mal((void**)&m->rows_d, sizeof(long long) * M);
-    mal((void**)&m->loss, sizeof(double));
-    mal((void**)&m->err, sizeof(int));
-    m->ws_floats = (size_t)32 * kOutPad * kIn;
+    mal((void**)&m->loss, kStatusBytes);
+    m->err = reinterpret_cast<int*>(m->loss + 1);
+    // partial sums of the four weight gradients together: each is split over K
+    // until its tiles of 128 x 64 times its K ranges reach two CTAs per SM
+    for (int l = 0; l < 4; ++l) {
+        size_t tiles = (size_t)(R[l] / 128) * (C[l] / 64);
+        while (tiles < 2 * 148) tiles *= 2;
+        m->ws_floats += tiles * 128 * 64;
+    }
     mal((void**)&m->ws, sizeof(float) * m->ws_floats);
     if (e != cudaSuccess) return mfail(m, OD_ERR_CUDA, std::string("od_mlp_create: ") + cudaGetErrorString(e));
     return OD_OK;
@@ -687,8 +922,8 @@ void od_mlp_destroy(od_mlp* m) {
     if (m->stream) cudaStreamSynchronize(m->stream);
     void* ps[] = {m->w, m->m1, m->m2, m->g, m->wb[0], m->wb[1], m->wb[2], m->wb[3], m->wbT[0], m->wbT[1], m->wbT[2],
                   m->wbT[3], m->Z[0], m->Z[1], m->Z[2], m->A[0], m->A[1], m->A[2], m->AT[0], m->AT[1], m->AT[2],
-                  m->Y, m->dY, m->dYT, m->dZa, m->dZaT, m->dZb, m->dZbT, m->X, m->XT, m->T, m->rows_d, m->loss,
-                  m->err, m->Xc, m->Yc, m->ws, m->wt};
+                  m->Y, m->dY, m->dYT, m->dZ[0], m->dZ[1], m->dZT[0], m->dZT[1], m->dZT[2], m->X, m->XT, m->T, m->rows_d, m->loss,
+                  m->Xc, m->Yc, m->ws, m->wt};
     for (void* p : ps)
         if (p) cudaFree(p);
     if (m->stream) cudaStreamDestroy(m->stream);
@@ -733,10 +968,10 @@ int od_mlp_get_params(od_mlp* m, float* host) {
 int od_mlp_forward(od_mlp* m, const void* X, int rows, float* Y) {
     if (!m || !X || !Y || rows <= 0 || rows % 128 || rows > m->mmax) return OD_ERR_ARG;
     cudaSetDevice(m->device);
-    cudaError_t e = cudaMemsetAsync(m->err, 0, sizeof(int), m->stream);
+    cudaError_t e = clear_status(m);
     if (e == cudaSuccess) e = forward(m, (const bf16*)X, rows, Y, false);
     if (e != cudaSuccess) return mfail(m, OD_ERR_CUDA, cudaGetErrorString(e));
-    return check_err(m);
+    return read_status(m, nullptr);
 }
 
 // Gradients (host fp32, flat layout) and loss of a batch given as device rows:
@@ -747,18 +982,17 @@ int od_mlp_gradients(od_mlp* m, const void* X, const void* XT, const float* T, i
     if (!m || !X || !XT || !T || rows <= 0 || rows % 128 || rows > m->mmax || valid <= 0 || valid > rows)
         return OD_ERR_ARG;
     cudaSetDevice(m->device);
-    cudaError_t e = cudaMemsetAsync(m->err, 0, sizeof(int), m->stream);
+    cudaError_t e = clear_status(m);
     if (e == cudaSuccess) e = cudaMemcpyAsync(m->T, T, sizeof(float) * (size_t)rows * kOutPad, cudaMemcpyDeviceToDevice, m->stream);
     if (e == cudaSuccess) e = forward(m, (const bf16*)X, rows, m->Y, true);
-    if (e == cudaSuccess) e = backward(m, (const bf16*)XT, rows, valid);
-    double l = 0;
-    if (e == cudaSuccess) e = cudaMemcpyAsync(&l, m->loss, sizeof(double), cudaMemcpyDeviceToHost, m->stream);
+    if (e == cudaSuccess) e = backward(m, (const bf16*)XT, rows, valid, nullptr);
     if (e == cudaSuccess && grads)
         e = cudaMemcpyAsync(grads, m->g, sizeof(float) * (size_t)m->nparam, cudaMemcpyDeviceToHost, m->stream);
-    if (e == cudaSuccess) e = cudaStreamSynchronize(m->stream);
     if (e != cudaSuccess) return mfail(m, OD_ERR_CUDA, cudaGetErrorString(e));
+    double l = 0;
+    const int rc = read_status(m, &l);
     if (loss) *loss = l / ((double)valid * kOut);
-    return check_err(m);
+    return rc;
 }
 
 // One Adam step on a batch gathered from device pools: features Xpool
@@ -769,35 +1003,43 @@ int od_mlp_train_step(od_mlp* m, const void* Xpool, const void* Tpool, const lon
     if (!m || !Xpool || !Tpool || !rows_host || batch <= 0 || batch > m->mmax) return OD_ERR_ARG;
     cudaSetDevice(m->device);
     const int M = (batch + 127) / 128 * 128;
-    cudaError_t e = cudaMemsetAsync(m->err, 0, sizeof(int), m->stream);
+    cudaError_t e = clear_status(m);
     if (e == cudaSuccess)
         e = cudaMemcpyAsync(m->rows_d, rows_host, sizeof(long long) * batch, cudaMemcpyHostToDevice, m->stream);
-    gather_kernel<<<blocks((long long)M * kIn, 256), 256, 0, m->stream>>>(
-        (const bf16*)Xpool, (const bf16*)Tpool, m->rows_d, batch, M, m->X, m->XT, m->T);
+    auto* gk = aligned16(Xpool) ? gather_kernel<true> : gather_kernel<false>;
+    gk<<<dim3(M / 64, kIn / 64), 256, 0, m->stream>>>((const bf16*)Xpool, m->rows_d, batch, M, m->X, m->XT);
     if (e == cudaSuccess) e = cudaGetLastError();
     if (e == cudaSuccess) e = forward(m, m->X, M, m->Y, true);
-    if (e == cudaSuccess) e = backward(m, m->XT, M, batch);
+    if (e == cudaSuccess) e = backward(m, m->XT, M, batch, (const bf16*)Tpool);
     m->step++;
     const float b1 = 0.9f, b2 = 0.999f, eps = 1e-8f;
     const float c1 = 1.f - std::pow(b1, (float)m->step), c2 = 1.f - std::pow(b2, (float)m->step);
-    for (int l = 0; l < 4 && e == cudaSuccess; ++l) {
-        const long long nw = (long long)m->rows[l] * m->cols[l];
-        adam_kernel<<<blocks(nw, 256), 256, 0, m->stream>>>(m->w + m->off_w[l], m->g + m->off_w[l], m->m1 + m->off_w[l],
-                                                              m->m2 + m->off_w[l], nw, lr, b1, b2, eps, c1, c2,
-                                                              m->rows[l], m->cols[l], m->wb[l], m->wbT[l]);
-        adam_kernel<<<blocks(m->rows[l], 256), 256, 0, m->stream>>>(m->w + m->off_b[l], m->g + m->off_b[l],
-                                                                     m->m1 + m->off_b[l], m->m2 + m->off_b[l],
-                                                                     m->rows[l], lr, b1, b2, eps, c1, c2, 1,
-                                                                     m->rows[l], nullptr, nullptr);
+    AdamArgs A{};
+    A.w = m->w;
+    A.m1 = m->m1;
+    A.m2 = m->m2;
+    A.g = m->g;
+    A.wt = m->wt;
+    A.p = {lr, b1, b2, eps, c1, c2};
+    int tiles = 0;
+    for (int l = 0; l < 4; ++l) {
+        A.off_w[l] = m->off_w[l];
+        A.off_b[l] = m->off_b[l];
+        A.rows[l] = m->rows[l];
+        A.cols[l] = m->cols[l];
+        A.wb[l] = m->wb[l];
+        A.wbT[l] = m->wbT[l];
+        tiles += (m->rows[l] / kAdamRows) * (m->cols[l] / 64);
+    }
+    if (e == cudaSuccess) {
+        adam_kernel<<<tiles + 4, 256, 0, m->stream>>>(A, tiles);
         e = cudaGetLastError();
     }
-    if (e == cudaSuccess) e = od::mlp::tile_fused_weights(m->wb, m->wt, m->stream);
-    double l = 0;
-    if (e == cudaSuccess) e = cudaMemcpyAsync(&l, m->loss, sizeof(double), cudaMemcpyDeviceToHost, m->stream);
-    if (e == cudaSuccess) e = cudaStreamSynchronize(m->stream);
     if (e != cudaSuccess) return mfail(m, OD_ERR_CUDA, cudaGetErrorString(e));
+    double l = 0;
+    const int rc = read_status(m, &l);
     if (loss) *loss = l / ((double)batch * kOut);
-    return check_err(m);
+    return rc;
 }
 
 // Normalisation of the closure's inputs and outputs.

@@ -14,13 +14,15 @@ namespace mlp {
 
 constexpr long long kSMs = 148;  // B200
 
-// out = sum of the ksplit partial tiles (+ bias)
-__global__ void splitk_reduce_kernel(const float* __restrict__ ws, int ks, long long mn, int N,
-                                     const float* __restrict__ bias, float* __restrict__ out) {
+// out = sum of the ksplit partial tiles in order (+ bias), a value per thread,
+// 16 loads in flight
+__global__ void __launch_bounds__(128) splitk_reduce_kernel(const float* __restrict__ ws, int ks, long long mn, int N,
+                                                            const float* __restrict__ bias, float* __restrict__ out) {
     const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= mn) return;
     float v = 0.f;
-    for (int z = 0; z < ks; ++z) v += ws[z * mn + i];
+#pragma unroll 16
+    for (int z = 0; z < ks; ++z) v += __ldcs(ws + z * mn + i);
     if (bias) v += bias[i % N];
     out[i] = v;
 }
@@ -42,11 +44,11 @@ cudaError_t launch_gemm_t(const GemmArgs& g, cudaStream_t s) {
     }
     const int ks = g.ksplit > 1 ? g.ksplit : 1;
     dim3 grid((unsigned)(g.M / BM), (unsigned)(g.N / NT), (unsigned)ks);
-    gemm_kernel<NT, EPI><<<grid, 128, smem, s>>>(g);
+    gemm_kernel<NT, EPI><<<grid, kGemmThreads, smem, s>>>(g);
     e = cudaGetLastError();
     if (e == cudaSuccess && ks > 1) {
         const long long mn = (long long)g.M * g.N;
-        splitk_reduce_kernel<<<(unsigned)((mn + 255) / 256), 256, 0, s>>>(g.ws, ks, mn, g.N, g.bias, g.out_f32);
+        splitk_reduce_kernel<<<(unsigned)((mn + 127) / 128), 128, 0, s>>>(g.ws, ks, mn, g.N, g.bias, g.out_f32);
         e = cudaGetLastError();
     }
     return e;
@@ -57,6 +59,63 @@ cudaError_t launch_nt(const GemmArgs& g, int nt, cudaStream_t s) {
     if (nt == 256) return launch_gemm_t<256, EPI>(g, s);
     if (nt == 128) return launch_gemm_t<128, EPI>(g, s);
     return launch_gemm_t<64, EPI>(g, s);
+}
+
+// K ranges of a product with few tiles: doubled until there are two CTAs per
+// SM, while every range keeps two K blocks and the partial sums fit.
+static int split_k(const GemmArgs& g, int nt, size_t ws_floats) {
+    const long long tiles = (long long)(g.M / BM) * (g.N / nt);
+    const int kblocks = g.K / BK;
+    int ks = 1;
+    while (tiles * ks < 2 * kSMs && kblocks % (2 * ks) == 0 && kblocks / (2 * ks) >= 2 &&
+           (size_t)(2 * ks) * g.M * g.N <= ws_floats)
+        ks *= 2;
+    return ks;
+}
+
+__global__ void __launch_bounds__(kGemmThreads, 2) gemm_group_kernel(const GemmGroup q) {
+    int i = 0;
+    while (i + 1 < kGroupMax && (int)blockIdx.x >= q.first[i + 1]) ++i;
+    const int t = (int)blockIdx.x - q.first[i], rows = q.g[i].M / BM, cols = q.g[i].N / 64;
+    gemm_tile<64, kStoreF32>(q.g[i], t % rows, t / rows % cols, t / (rows * cols));
+}
+
+// n <= kGroupMax fp32 products (no bias) in one launch, each split over K as
+// launch_gemm splits it; ksplit of each is set, and where it is above 1 its
+// partial sums are left in the product's own part of ws (the caller adds
+// them up). The weight gradients of the closure: four products of 3 to 28
+// tiles, 51 us launched one by one at a batch of 8192 (11 to 17 each), 40
+// together.
+cudaError_t launch_gemm_group(GemmArgs* g, int n, float* ws, size_t ws_floats, cudaStream_t s) {
+    if (n < 1 || n > kGroupMax) return cudaErrorInvalidValue;
+    GemmGroup q{};
+    size_t used = 0;
+    int ctas = 0;
+    for (int i = 0; i < n; ++i) {
+        GemmArgs& a = g[i];
+        if (a.M <= 0 || a.N <= 0 || a.K <= 0 || a.M % BM || a.N % 64 || a.K % BK || a.bias)
+            return cudaErrorInvalidValue;
+        a.ws = ws + used;
+        a.ksplit = split_k(a, 64, ws_floats - used);
+        if (a.ksplit > 1) used += (size_t)a.ksplit * a.M * a.N;
+        q.g[i] = a;
+        q.first[i] = ctas;
+        ctas += (a.M / BM) * (a.N / 64) * a.ksplit;
+    }
+    for (int i = n; i <= kGroupMax; ++i) q.first[i] = ctas;
+    const size_t smem = gemm_smem_bytes<64>();
+    static bool prepared[64] = {};
+    int dev = 0;
+    cudaError_t e = cudaGetDevice(&dev);
+    if (e != cudaSuccess) return e;
+    if (dev < 0 || dev >= 64) return cudaErrorInvalidDevice;
+    if (!prepared[dev]) {
+        e = cudaFuncSetAttribute(gemm_group_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        if (e != cudaSuccess) return e;
+        prepared[dev] = true;
+    }
+    gemm_group_kernel<<<(unsigned)ctas, kGemmThreads, smem, s>>>(q);
+    return cudaGetLastError();
 }
 
 // C = A B^T with the epilogue `epi`; M % 128 == 0, N % 64 == 0, K % 64 == 0.
@@ -75,16 +134,7 @@ cudaError_t launch_gemm(const GemmArgs& g0, int epi, cudaStream_t s, size_t ws_f
             break;
         }
     }
-    g.ksplit = 1;
-    if (epi == kStoreF32 && g.ws) {
-        const long long tiles = rows * (g.N / nt);
-        const int kblocks = g.K / BK;
-        int ks = 1;
-        while (tiles * ks < 2 * kSMs && kblocks % (2 * ks) == 0 && kblocks / (2 * ks) >= 2 &&
-               (size_t)(2 * ks) * g.M * g.N <= ws_floats)
-            ks *= 2;
-        g.ksplit = ks;
-    }
+    g.ksplit = epi == kStoreF32 && g.ws ? split_k(g, nt, ws_floats) : 1;
     switch (epi) {
         case kStoreF32: return launch_nt<kStoreF32>(g, nt, s);
         case kBiasGelu: return launch_nt<kBiasGelu>(g, nt, s);
