@@ -2,6 +2,8 @@
 // od_inst_*.cu translation units only.
 #pragma once
 
+#include <type_traits>
+
 #include "od_launch.h"
 #include "od_stage.cuh"
 
@@ -49,6 +51,10 @@ cudaError_t launch_a_epb(const StageAParams<S, P, C>& A, long long nelem, int ep
     if (epb == 2 && !feat) return launch_a<S, P, C, M, FLUX, 2>(A, nelem, s);
     return launch_a<S, P, C, M, FLUX, 4>(A, nelem, s, feat);
 }
+
+// f32 fluxes under an f64 state: the policy that keeps their operation order
+template <class S, class C, class M>
+using MathFor = std::conditional_t<sizeof(S) == 8 && sizeof(C) == 4, WideState<M>, M>;
 
 template <class S, class P, class C, class M>
 cudaError_t launch_a_flux(const StageAParams<S, P, C>& A, int flux, long long nelem, int epb, cudaStream_t s,
@@ -105,6 +111,7 @@ cudaError_t launch_stage_t(const StageLaunch& L, cudaStream_t s) {
     A.m.nelem = L.nelem;
     mesh_set_div(A.m);
     A.m.npts = L.nelem * NE;
+    A.kappa = heat_coeff_host<C>((C)L.mu);
     A.tp = cast_tab<P>(L.tab);
     A.tc = cast_tab<C>(L.tab);
     for (int d = 0; d < 3; ++d) A.jac[d] = (C)L.jac[d];
@@ -113,7 +120,6 @@ cudaError_t launch_stage_t(const StageLaunch& L, cudaStream_t s) {
     A.rb = (P)L.rb;
     A.rc = (P)L.rc;
     A.mu = (C)L.mu;
-    A.kappa = heat_coeff_host<C>(A.mu);
     A.forcing = (C)L.forcing;
     A.suth = (C)L.suth;
     A.flux = L.flux;
@@ -128,11 +134,11 @@ cudaError_t launch_stage_t(const StageLaunch& L, cudaStream_t s) {
         if (L.ev[0]) cudaEventRecord(L.ev[0], s);
         if constexpr (has_fast_variant<C>()) {
             if (L.fast_math)
-                err = launch_a_flux<S, P, C, MathFast>(A, L.flux, count, L.epb_a, s, feat);
+                err = launch_a_flux<S, P, C, MathFor<S, C, MathFast>>(A, L.flux, count, L.epb_a, s, feat);
             else
-                err = launch_a_flux<S, P, C, MathIeee>(A, L.flux, count, L.epb_a, s, feat);
+                err = launch_a_flux<S, P, C, MathFor<S, C, MathIeee>>(A, L.flux, count, L.epb_a, s, feat);
         } else {
-            err = launch_a_flux<S, P, C, MathIeee>(A, L.flux, count, L.epb_a, s, feat);
+            err = launch_a_flux<S, P, C, MathFor<S, C, MathIeee>>(A, L.flux, count, L.epb_a, s, feat);
         }
         if (err != cudaSuccess) return err;
         if (L.ev[1]) cudaEventRecord(L.ev[1], s);
@@ -192,9 +198,9 @@ cudaError_t prepare_m() {
 
 template <class S, class P, class C>
 cudaError_t prepare_t() {
-    cudaError_t e = prepare_m<S, P, C, MathIeee>();
+    cudaError_t e = prepare_m<S, P, C, MathFor<S, C, MathIeee>>();
     if constexpr (has_fast_variant<C>()) {
-        if (e == cudaSuccess) e = prepare_m<S, P, C, MathFast>();
+        if (e == cudaSuccess) e = prepare_m<S, P, C, MathFor<S, C, MathFast>>();
     }
     return e;
 }

@@ -27,6 +27,7 @@ enum Flux : int { kSlau2 = 0, kAusmPlus = 1, kRusanov = 2 };
 // --use_fast_math build; f64 operands stay IEEE (fast math does not touch them).
 struct MathIeee {
     static constexpr bool kSutherland = false;
+    static constexpr bool kWideState = false;
     template <class T>
     static __device__ __forceinline__ T rcp(T x) { return (T)1.0 / x; }
     template <class T>
@@ -37,6 +38,7 @@ struct MathIeee {
 
 struct MathFast {
     static constexpr bool kSutherland = false;
+    static constexpr bool kWideState = false;
     template <class T>
     static __device__ __forceinline__ T rcp(T x) {
         if constexpr (sizeof(T) == 4) {
@@ -71,6 +73,16 @@ struct WithSutherland : Base {
     static constexpr bool kSutherland = true;
 };
 
+// A math policy for f32 flux arithmetic under an f64 state (the u64/c32 and
+// mixed pipelines). Such a state shows every rounding of the fluxes (at 1e-8,
+// where an f32 state rounds them away), so these pipelines keep the formulas'
+// operation order that their states, checkpoints and restarts have always
+// had; the other pipelines take the forms with fewer operations.
+template <class Base>
+struct WideState : Base {
+    static constexpr bool kWideState = true;
+};
+
 template <class C>
 struct Gas {
     static __device__ __forceinline__ C gamma() { return (C)1.4; }
@@ -93,28 +105,41 @@ __device__ __forceinline__ P raw_pressure(P r, P m0, P m1, P m2, P E) {
 template <class C>
 __device__ __forceinline__ C clamp_p(C p) { return cmax((C)1e-7, p); }
 
-// Face state in compute type: conserved variables, 1/rho, velocity and the
-// clamped pressure (recovered in the state precision P by the caller).
+// State of a point in compute type: conserved variables, 1/rho, velocity, the
+// clamped pressure, and what the viscous flux needs: kinetic and internal
+// energy per volume, or (kWideState) the unclamped pressure.
 template <class C>
 struct FaceState {
     C q[5];
     C ir;
     C vel[3];
-    C p;   // clamped
+    C ke;     // |m|^2 / (2 rho)
+    C ein;    // E - ke
+    C praw;   // (gamma - 1) ein
+    C p;      // praw clamped (the inviscid fluxes and sound speeds)
 };
 
+// kWideState: the pressure recovered in the state arithmetic's precision P.
+// Otherwise the kinetic energy comes from the velocity (one reciprocal per
+// point, no second division).
 template <class M, class C, class P>
-__device__ __forceinline__ FaceState<C> make_face_state(const P* qp, C& praw_out) {
+__device__ __forceinline__ FaceState<C> make_face_state(const P* qp) {
     FaceState<C> s;
 #pragma unroll
     for (int v = 0; v < 5; ++v) s.q[v] = (C)qp[v];
-    P praw = raw_pressure<M, P>(qp[0], qp[1], qp[2], qp[3], qp[4]);
-    praw_out = (C)praw;
-    s.p = clamp_p<C>((C)praw);
+    if constexpr (M::kWideState) {
+        s.praw = (C)raw_pressure<M, P>(qp[0], qp[1], qp[2], qp[3], qp[4]);
+        s.p = clamp_p<C>(s.praw);
+    }
     s.ir = M::rcp(s.q[0]);
     s.vel[0] = s.q[1] * s.ir;
     s.vel[1] = s.q[2] * s.ir;
     s.vel[2] = s.q[3] * s.ir;
+    if constexpr (!M::kWideState) {
+        s.ke = (C)0.5 * (s.q[1] * s.vel[0] + s.q[2] * s.vel[1] + s.q[3] * s.vel[2]);
+        s.ein = s.q[4] - s.ke;
+        s.p = clamp_p<C>(Gas<C>::gm1() * s.ein);
+    }
     return s;
 }
 
@@ -130,21 +155,16 @@ __device__ __forceinline__ void euler_flux(const FaceState<C>& s, C* f) {
     f[4] = vn * (s.q[4] + s.p);
 }
 
-// Inviscid flux along axis d (d known after unrolling).
-template <class C>
-__device__ __forceinline__ void euler_flux_dyn(const FaceState<C>& s, int d, C* f) {
-    C vn = s.vel[d];
-    f[0] = s.q[1 + d];
-    f[1] = s.q[1] * vn;
-    f[2] = s.q[2] * vn;
-    f[3] = s.q[3] * vn;
-    f[1 + d] += s.p;
-    f[4] = vn * (s.q[4] + s.p);
-}
-
+// sqrt(gamma p / max(rho, 1e-7)); not kWideState: with the reciprocal of rho
+// at hand (NaN for a NaN density)
 template <class M, class C>
-__device__ __forceinline__ C sound_speed(C p, C r) {
-    return M::sqrt(cmax((C)0.0, M::div(Gas<C>::gamma() * p, cmax((C)1e-7, r))));
+__device__ __forceinline__ C sound_speed(const FaceState<C>& s) {
+    if constexpr (M::kWideState) {
+        return M::sqrt(cmax((C)0.0, M::div(Gas<C>::gamma() * s.p, cmax((C)1e-7, s.q[0]))));
+    } else {
+        const C ir = (C)1e-7 > s.q[0] ? (C)1e7 : s.ir;
+        return M::sqrt(cmax((C)0.0, Gas<C>::gamma() * s.p * ir));
+    }
 }
 
 // Dynamic viscosity at a point. Policies without kSutherland: constant mu
@@ -163,7 +183,100 @@ __device__ __forceinline__ C viscosity(C mu, C suth, const FaceState<C>& s) {
     }
 }
 
-// Heat-flux coefficient mu gamma / (Pr (gamma - 1)), in the reference's
+// The viscous terms, arranged so that every factor 1/rho is applied once.
+// With w_ab = d(rho u_a)/dx_b - u_a d(rho)/dx_b = rho du_a/dx_b:
+//   tau_ab = (mu / rho) (w_ab + w_ba - 2/3 delta_ab tr w)
+// and the heat flux -mu gamma / (Pr (gamma - 1)) d(p/rho)/dx_b, p = (gamma - 1)
+// ein, whose gradient needs no pressure:
+//   -heat_b = (mu / rho) (gamma / Pr)
+//             (dE/dx_b - u . d(rho u)/dx_b + (ke - ein) / rho d(rho)/dx_b)
+// 28 operations a face and 77 a point for all three directions (with every
+// velocity gradient, pressure gradient and kinetic-energy gradient formed on
+// its own: about 45 and 150). With the one reciprocal per point, the shared
+// flux rows and the folded jumps: phase A 1948 -> 1779 warp instructions per
+// element in f32 (85.1 -> 82.1 us at 32^3), 269 -> 243 us in f64.
+
+// the bracket of -heat_b; ce = (ke - ein) / rho
+template <class C>
+__device__ __forceinline__ C heat_bracket(const FaceState<C>& s, const C* g, C ce, int b) {
+    return g[12 + b] + ce * g[b] - s.vel[0] * g[3 + b] - s.vel[1] * g[6 + b] - s.vel[2] * g[9 + b];
+}
+
+template <class C>
+__device__ __forceinline__ constexpr C gamma_over_pr() { return (C)(1.4 / 0.72); }
+
+// Viscous flux along axis D at a face point from the state and the
+// 15-component conserved gradient g[3*var + axis] (only the 11 components
+// the D-flux reads are touched).
+template <int D, class C>
+__device__ __forceinline__ void viscous_flux(const FaceState<C>& s, const C* g, C mu, C* f) {
+    auto w = [&](int a, int b) -> C { return g[3 * (1 + a) + b] - s.vel[a] * g[b]; };
+    const C mi = mu * s.ir;
+    const C tr = (w(0, 0) + w(1, 1) + w(2, 2)) * ((C)2.0 / (C)3.0);
+    C tau[3];
+#pragma unroll
+    for (int a = 0; a < 3; ++a) {
+        if (a == D)
+            tau[a] = mi * ((C)2.0 * w(D, D) - tr);
+        else
+            tau[a] = mi * (w(a, D) + w(D, a));
+    }
+    f[0] = (C)0.0;
+    f[1] = tau[0];
+    f[2] = tau[1];
+    f[3] = tau[2];
+    f[4] = mi * gamma_over_pr<C>() * heat_bracket(s, g, (s.ke - s.ein) * s.ir, D) + s.vel[0] * tau[0] +
+           s.vel[1] * tau[1] + s.vel[2] * tau[2];
+}
+
+// Volume fluxes F_euler - F_viscous of all three directions at a solution
+// point. The momentum fluxes rho u_a u_b + p delta_ab - tau_ab are symmetric
+// (m[a][b], b >= a); the mass flux along d is the momentum q[1 + d].
+template <class C>
+struct VolumeFluxes {
+    C m00, m11, m22, m01, m02, m12;
+    C e[3];
+};
+
+template <class C>
+__device__ __forceinline__ VolumeFluxes<C> volume_fluxes(const FaceState<C>& s, const C* g, C mu) {
+    auto w = [&](int a, int b) -> C { return g[3 * (1 + a) + b] - s.vel[a] * g[b]; };
+    const C mi = mu * s.ir;
+    const C w00 = w(0, 0), w11 = w(1, 1), w22 = w(2, 2);
+    const C tr = (w00 + w11 + w22) * ((C)2.0 / (C)3.0);
+    const C t00 = mi * ((C)2.0 * w00 - tr), t11 = mi * ((C)2.0 * w11 - tr), t22 = mi * ((C)2.0 * w22 - tr);
+    const C t01 = mi * (w(0, 1) + w(1, 0)), t02 = mi * (w(0, 2) + w(2, 0)), t12 = mi * (w(1, 2) + w(2, 1));
+    const C u = s.vel[0], v = s.vel[1], x = s.vel[2];
+    VolumeFluxes<C> f;
+    f.m00 = s.q[1] * u - t00 + s.p;
+    f.m11 = s.q[2] * v - t11 + s.p;
+    f.m22 = s.q[3] * x - t22 + s.p;
+    f.m01 = s.q[1] * v - t01;
+    f.m02 = s.q[1] * x - t02;
+    f.m12 = s.q[2] * x - t12;
+    const C h = s.q[4] + s.p, ce = (s.ke - s.ein) * s.ir, k = mi * gamma_over_pr<C>();
+    f.e[0] = h * u - k * heat_bracket(s, g, ce, 0) - u * t00 - v * t01 - x * t02;
+    f.e[1] = h * v - k * heat_bracket(s, g, ce, 1) - u * t01 - v * t11 - x * t12;
+    f.e[2] = h * x - k * heat_bracket(s, g, ce, 2) - u * t02 - v * t12 - x * t22;
+    return f;
+}
+
+// ---- the viscous terms of the kWideState pipelines, in the reference's order
+// (device_functions.cuh)
+
+// Inviscid flux along axis d (d known after unrolling).
+template <class C>
+__device__ __forceinline__ void euler_flux_dyn(const FaceState<C>& s, int d, C* f) {
+    C vn = s.vel[d];
+    f[0] = s.q[1 + d];
+    f[1] = s.q[1] * vn;
+    f[2] = s.q[2] * vn;
+    f[3] = s.q[3] * vn;
+    f[1 + d] += s.p;
+    f[4] = vn * (s.q[4] + s.p);
+}
+
+// kWideState: heat-flux coefficient mu gamma / (Pr (gamma - 1)), in the reference's
 // operation order (device_functions.cuh:44). Constant viscosity: the value
 // formed once per launch on the host with the same IEEE operations
 // (kappa_const, heat_coeff_host); Sutherland's law: per point.
@@ -180,11 +293,9 @@ __host__ inline C heat_coeff_host(C mu) {
     return mu * (C)1.4 / ((C)0.72 * ((C)1.4 - (C)1.0));
 }
 
-// Viscous flux along axis D at a face point from the state and the
-// 15-component conserved gradient g[3*var + axis] (only the 11 components
-// the D-flux reads are touched); kappa = heat_coeff(mu).
+// Viscous flux along axis D at a face point (see viscous_flux).
 template <int D, class C>
-__device__ __forceinline__ void viscous_flux(const FaceState<C>& s, C praw, const C* g, C mu, C kappa, C* f) {
+__device__ __forceinline__ void viscous_flux_wide(const FaceState<C>& s, const C* g, C mu, C kappa, C* f) {
     const C ir = s.ir;
     // d(vel_a)/d(x_b) for the pairs the D-flux needs
     auto dv = [&](int a, int b) -> C { return (g[3 * (1 + a) + b] - s.vel[a] * g[b]) * ir; };
@@ -200,7 +311,7 @@ __device__ __forceinline__ void viscous_flux(const FaceState<C>& s, C praw, cons
     C ke = (C)0.5 * (s.q[1] * s.vel[0] + s.q[2] * s.vel[1] + s.q[3] * s.vel[2]);
     C dke = (s.q[1] * g[3 + D] + s.q[2] * g[6 + D] + s.q[3] * g[9 + D]) * ir - ke * g[D] * ir;
     C dp = Gas<C>::gm1() * (g[12 + D] - dke);
-    C heat = -kappa * (dp * ir - praw * g[D] * ir * ir);
+    C heat = -kappa * (dp * ir - s.praw * g[D] * ir * ir);
     f[0] = (C)0.0;
     f[1] = tau[0];
     f[2] = tau[1];
@@ -209,11 +320,9 @@ __device__ __forceinline__ void viscous_flux(const FaceState<C>& s, C praw, cons
 }
 
 // Volume fluxes of all three directions at a solution point:
-// out[d][v] = F_euler,d - F_viscous,d. The velocity gradient, stress tensor
-// and heat flux are formed once and shared by the three directions.
+// out[d][v] = F_euler,d - F_viscous,d.
 template <class C>
-__device__ __forceinline__ void volume_fluxes(const FaceState<C>& s, C praw, const C* g, C mu, C kappa,
-                                              C out[3][5]) {
+__device__ __forceinline__ void volume_fluxes_wide(const FaceState<C>& s, const C* g, C mu, C kappa, C out[3][5]) {
     const C ir = s.ir;
     C dvel[3][3];
 #pragma unroll
@@ -238,7 +347,7 @@ __device__ __forceinline__ void volume_fluxes(const FaceState<C>& s, C praw, con
         C vn = s.vel[d];
         C dke = (s.q[1] * g[3 + d] + s.q[2] * g[6 + d] + s.q[3] * g[9 + d]) * ir - ke * g[d] * ir;
         C dp = Gas<C>::gm1() * (g[12 + d] - dke);
-        C heat = -kappa * (dp * ir - praw * g[d] * ir * ir);
+        C heat = -kappa * (dp * ir - s.praw * g[d] * ir * ir);
         // (F_euler) - (F_viscous), each formed first as the reference does
         C fe[5];
         euler_flux_dyn(s, d, fe);
@@ -255,7 +364,7 @@ __device__ __forceinline__ void volume_fluxes(const FaceState<C>& s, C praw, con
 template <class M, int D, class C>
 __device__ __forceinline__ void rusanov(const FaceState<C>& L, const FaceState<C>& R, C* f) {
     C vnL = L.vel[D], vnR = R.vel[D];
-    C smax = cmax(fabs(vnL) + sound_speed<M>(L.p, L.q[0]), fabs(vnR) + sound_speed<M>(R.p, R.q[0]));
+    C smax = cmax(fabs(vnL) + sound_speed<M>(L), fabs(vnR) + sound_speed<M>(R));
     C fL[5], fR[5];
     euler_flux<D>(L, fL);
     euler_flux<D>(R, fR);
@@ -266,7 +375,7 @@ __device__ __forceinline__ void rusanov(const FaceState<C>& L, const FaceState<C
 template <class M, int D, class C>
 __device__ __forceinline__ void ausm_plus(const FaceState<C>& L, const FaceState<C>& R, C* f) {
     const C alpha = (C)0.1875, beta = (C)0.125;
-    C cm = cmax(sound_speed<M>(L.p, L.q[0]), sound_speed<M>(R.p, R.q[0]));
+    C cm = cmax(sound_speed<M>(L), sound_speed<M>(R));
     C icm = M::rcp(cm);
     C mL = L.vel[D] * icm, mR = R.vel[D] * icm;
     C mp, pp, mm, pm;
@@ -305,7 +414,7 @@ __device__ __forceinline__ void slau2(const FaceState<C>& L, const FaceState<C>&
     C vnL = L.vel[D], vnR = R.vel[D];
     C q2L = L.vel[0] * L.vel[0] + L.vel[1] * L.vel[1] + L.vel[2] * L.vel[2];
     C q2R = R.vel[0] * R.vel[0] + R.vel[1] * R.vel[1] + R.vel[2] * R.vel[2];
-    C cf = (C)0.5 * (sound_speed<M>(L.p, rL) + sound_speed<M>(R.p, rR));
+    C cf = (C)0.5 * (sound_speed<M>(L) + sound_speed<M>(R));
     C icf = M::rcp(cf);
     C mL = vnL * icf, mR = vnR * icf;
     C qbar = M::sqrt((C)0.5 * (q2L + q2R));

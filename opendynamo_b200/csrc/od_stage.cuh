@@ -75,25 +75,33 @@ struct Tab {
     T gR[4];   // Radau g_R'(x_a)
 };
 
-// The operators of each direction scaled by its Jacobian 2/h, so that the
-// corrected gradient, the divergence and the lifting are pure FMA chains:
-// d[dir][a*4+m] = D[a*4+m] jac[dir], gl / gr[dir][a] = g_L' / g_R'(x_a) jac[dir]
-// (products rounded in T).
+// The operators of each direction scaled by its Jacobian 2/h (products
+// rounded in T), with the signs and halves of their uses folded in, so that
+// the corrected gradient, the divergence and the lifting are pure FMA chains:
+//   d[dir][a*4+m] = D[a*4+m] jac        gradient
+//   hl / hr[dir][a] = g_L' / g_R'(x_a) jac / 2   times the jump at the face
+//   nd = -d                              divergence
+//   nl / nr = -g_L' / g_R' jac           lifting
 template <class T>
 struct ScaledTab {
-    T d[3][16];
-    T gl[3][4];
-    T gr[3][4];
+    T d[3][16], nd[3][16];
+    T hl[3][4], hr[3][4];
+    T nl[3][4], nr[3][4];
 };
 
 template <class T, class TabT>
 __host__ ScaledTab<T> scale_tab(const TabT& t, const T* jac) {
     ScaledTab<T> r;
     for (int dir = 0; dir < 3; ++dir) {
-        for (int i = 0; i < 16; ++i) r.d[dir][i] = (T)(t.D[i] * jac[dir]);
+        for (int i = 0; i < 16; ++i) {
+            r.d[dir][i] = (T)(t.D[i] * jac[dir]);
+            r.nd[dir][i] = -r.d[dir][i];
+        }
         for (int a = 0; a < 4; ++a) {
-            r.gl[dir][a] = (T)(t.gL[a] * jac[dir]);
-            r.gr[dir][a] = (T)(t.gR[a] * jac[dir]);
+            r.nl[dir][a] = -(T)(t.gL[a] * jac[dir]);
+            r.nr[dir][a] = -(T)(t.gR[a] * jac[dir]);
+            r.hl[dir][a] = (T)-0.5 * r.nl[dir][a];
+            r.hr[dir][a] = (T)-0.5 * r.nr[dir][a];
         }
     }
     return r;
@@ -169,20 +177,6 @@ template <class T, class CL, class CR>
 __device__ __forceinline__ void trace4_lr(const T* q, const CL& cL, const CR& cR, T& oL, T& oR) {
     oL = trace4(q, cL);
     oR = trace4(q, cR);
-}
-
-// r[a] = sum_m D[a*4+m] q[m] for a = 0..3 (the FR derivative along a line,
-// D already scaled by the Jacobian). Paired f32 forms (FFMA2) of these loops
-// measured 3% slower on B200: the pairs cost operand moves and registers.
-template <class T, class DM>
-__device__ __forceinline__ void deriv4(const T* q, const DM& D, T* r) {
-#pragma unroll
-    for (int a = 0; a < 4; ++a) {
-        T df = D[a * 4] * q[0];
-#pragma unroll
-        for (int mm = 1; mm < 4; ++mm) df = fma(D[a * 4 + mm], q[mm], df);
-        r[a] = df;
-    }
 }
 
 // Sum over the four lanes of an aligned lane group (4g .. 4g+3) of p[q], for
@@ -330,7 +324,7 @@ struct StageAParams {
     P ra, rb, rc;
     C mu, forcing;
     C suth;             // Sutherland S = s_suth / t_ref, < 0: constant mu
-    C kappa;            // heat-flux coefficient of the constant mu (heat_coeff_host)
+    C kappa;            // kWideState: heat-flux coefficient of the constant mu (heat_coeff_host)
     int flags;
     int flux;           // scheme id, read when the kernel's FLUX is kFluxRuntime
     long long e0, e1;   // element range of this launch
@@ -389,7 +383,7 @@ __device__ __forceinline__ void stage_a_features(const PA& A, SlotA<P, C>& sm, l
             st[c * 64 + p] =
                 __float2bfloat16_rn(fminf(fmaxf((ch[c] - fp.mean[c]) * fp.inv_scale[c], -kFeatClip), kFeatClip));
     }
-    __syncthreads();
+    __syncwarp();
     if (live) {
         // tile (e / 128), channel c: a 128 x 64 block, row e % 128, 16-byte
         // chunk kc at ((row / 8) * 1024 + kc * 128 + (row % 8) * 16) bytes
@@ -401,7 +395,7 @@ __device__ __forceinline__ void stage_a_features(const PA& A, SlotA<P, C>& sm, l
                 *reinterpret_cast<const uint4*>(&st[c * 64 + 8 * kc]);
         }
     }
-    __syncthreads();   // the gradient rows are P2's from here
+    __syncwarp();   // the gradient rows are P2's from here
 }
 
 // Inviscid part of the face corrections at the two faces of a line. Each
@@ -427,8 +421,7 @@ __device__ __forceinline__ void minus_face(const FaceState<C>& so, const P* nbr,
         wall_face<M, D, P, C>(so, fe, j);
         return;
     }
-    C praw;
-    FaceState<C> sn = make_face_state<M, C, P>(nbr, praw);
+    const FaceState<C> sn = make_face_state<M, C, P>(nbr);
     if constexpr (FLUX == kFluxRuntime)
         interface_flux_rt<M, D>(rflux, sn, so, fi);
     else
@@ -500,15 +493,18 @@ __device__ __forceinline__ void row_line_store(T* row, const LineIdx& li, const 
 // interface flux solved in the line pass), Fv_own (components 1..4) at a
 // plus face.
 // REG: the face's correction j is in registers (jreg), else in shared memory.
-// s, praw: the face state (make_face_state of the face values).
+// s: the face state (make_face_state of the face values).
 template <class M, int D, bool REG, class PA, class P = typename PA::P_t, class C = typename PA::C_t>
 __device__ __forceinline__ void viscous_face(const PA& A, SlotA<P, C>& sm, long long e, int l, int side,
-                                             const FaceState<C>& s, C praw, const C* gt, bool live, C* jreg,
+                                             const FaceState<C>& s, const C* gt, bool live, C* jreg,
                                              const C* fi) {
     const int f = 2 * D + side;
     C fv[NV];
     const C mu = viscosity<M>(A.mu, A.suth, s);
-    viscous_flux<D>(s, praw, gt, mu, heat_coeff<M>(mu, A.kappa), fv);
+    if constexpr (M::kWideState)
+        viscous_flux_wide<D>(s, gt, mu, heat_coeff<M>(mu, A.kappa), fv);
+    else
+        viscous_flux<D>(s, gt, mu, fv);
 #pragma unroll
     for (int v = 0; v < NV; ++v) {
         if constexpr (REG)
@@ -611,17 +607,26 @@ __device__ __forceinline__ void line_pass(const PA& A, SlotA<P, C>& sm, long lon
         }
     }
     }
-    // corrected gradient along the line (BR1): jl g_L' + jr g_R' + D q, all
-    // scaled by the Jacobian, as one FMA chain per point
+    // corrected gradient along the line (BR1): the jump to the common value is
+    // half the difference across the face; (n_L - o_L) g_L'/2 + (n_R - o_R)
+    // g_R'/2 + D q, all scaled by the Jacobian, as one FMA chain per point
+    // (kWideState: the jump formed from the common value, times g_L', g_R')
     C gnL[NV], gnR[NV];   // z pass: face values of the normal gradient components
 #pragma unroll
     for (int v = 0; v < NV; ++v) {
-        const C jl = (C)((P)0.5 * (nL[v] + oL[v]) - oL[v]);
-        const C jr = (C)((P)0.5 * (nR[v] + oR[v]) - oR[v]);
+        C jl, jr;
+        if constexpr (M::kWideState) {
+            jl = (C)((P)0.5 * (nL[v] + oL[v]) - oL[v]);
+            jr = (C)((P)0.5 * (nR[v] + oR[v]) - oR[v]);
+        } else {
+            jl = (C)(nL[v] - oL[v]);
+            jr = (C)(nR[v] - oR[v]);
+        }
         C gv[4];
 #pragma unroll
         for (int a = 0; a < 4; ++a) {
-            C gg = fma(jr, A.sc.gr[D][a], jl * A.sc.gl[D][a]);
+            C gg = M::kWideState ? fma(-jr, A.sc.nr[D][a], -jl * A.sc.nl[D][a])
+                                 : fma(jr, A.sc.hr[D][a], jl * A.sc.hl[D][a]);
 #pragma unroll
             for (int mm = 0; mm < 4; ++mm) gg = fma(A.sc.d[D][a * 4 + mm], (C)q[v][mm], gg);
             if constexpr (sizeof(C) == 8) {
@@ -635,9 +640,8 @@ __device__ __forceinline__ void line_pass(const PA& A, SlotA<P, C>& sm, long lon
     // inviscid parts at the two faces of this line; F_I stays in registers
     // until the minus face's viscous flux is known (P5)
     C j0[NV], j1[NV];
-    C prawL, prawR;
-    const FaceState<C> sL = make_face_state<M, C, P>(oL, prawL);
-    const FaceState<C> sR = make_face_state<M, C, P>(oR, prawR);
+    const FaceState<C> sL = make_face_state<M, C, P>(oL);
+    const FaceState<C> sR = make_face_state<M, C, P>(oR);
     minus_face<M, FLUX, D, P, C>(sL, nL, D == 1 && nb0 < 0, j0, fi, A.flux);
     plus_face<M, D, P, C>(sR, D == 1 && nb1 < 0, j1);
     if constexpr (D == 2) {
@@ -658,8 +662,8 @@ __device__ __forceinline__ void line_pass(const PA& A, SlotA<P, C>& sm, long lon
                 trace4_lr(w, A.tc.eL, A.tc.eR, gL[c], gR[c]);
             }
         }
-        viscous_face<M, 2, true>(A, sm, e, l, 0, sL, prawL, gL, live, j0, fi);
-        viscous_face<M, 2, true>(A, sm, e, l, 1, sR, prawR, gR, live, j1, fi);
+        viscous_face<M, 2, true>(A, sm, e, l, 0, sL, gL, live, j0, fi);
+        viscous_face<M, 2, true>(A, sm, e, l, 1, sR, gR, live, j1, fi);
     }
 #pragma unroll
     for (int v = 0; v < NV; ++v) {
@@ -722,14 +726,28 @@ __device__ __forceinline__ void face_grad_pass(const PA& A, SlotA<P, C>& sm, lon
         }
     }
     if (!wall0) {
-        C praw;
-        const FaceState<C> st = make_face_state<M, C, P>(qL, praw);
-        viscous_face<M, D, D == 0>(A, sm, e, l, 0, st, praw, gL, live, jx[0], fi);
+        const FaceState<C> st = make_face_state<M, C, P>(qL);
+        viscous_face<M, D, D == 0>(A, sm, e, l, 0, st, gL, live, jx[0], fi);
     }
     if (!wall1) {
-        C praw;
-        const FaceState<C> st = make_face_state<M, C, P>(qR, praw);
-        viscous_face<M, D, D == 0>(A, sm, e, l, 1, st, praw, gR, live, jx[1], fi);
+        const FaceState<C> st = make_face_state<M, C, P>(qR);
+        viscous_face<M, D, D == 0>(A, sm, e, l, 1, st, gR, live, jx[1], fi);
+    }
+}
+
+// Rows of the dead gradient that hold F_y and F_z between P6 and P7. F_y of
+// rho w is F_z of rho v, and the mass fluxes are the momenta, read from the
+// state (kWideState: all ten fluxes in rows 0-9).
+constexpr int kFy1 = 0, kFy2 = 1, kFy3 = 2, kFy4 = 3, kFz1 = 4, kFz2 = kFy3, kFz3 = 5, kFz4 = 6;
+
+template <class M, int D, class P, class C>
+__device__ __forceinline__ const C* flux_row(const SlotA<P, C>& sm, int v) {
+    if constexpr (M::kWideState) {
+        return sm.g[(D == 1 ? 0 : 5) + v];
+    } else if constexpr (D == 1) {
+        return v == 0 ? sm.u[2] : sm.g[v == 1 ? kFy1 : v == 2 ? kFy2 : v == 3 ? kFy3 : kFy4];
+    } else {
+        return v == 0 ? sm.u[3] : sm.g[v == 1 ? kFz1 : v == 2 ? kFz2 : v == 3 ? kFz3 : kFz4];
     }
 }
 
@@ -743,45 +761,61 @@ __device__ __forceinline__ void face_grad_pass(const PA& A, SlotA<P, C>& sm, lon
 // of the same plane / column load the same line: broadcasts), so no pass
 // along y and z lines and no barrier before the update. Operation order per
 // point as a derivative along the line: D[a][0] F_0, then FMAs for m = 1..3.
-template <class PA, class P = typename PA::P_t, class C = typename PA::C_t>
+template <class M, class PA, class P = typename PA::P_t, class C = typename PA::C_t>
 __device__ __forceinline__ void stage_a_update(const PA& A, SlotA<P, C>& sm, long long ec, int l, int swz,
                                                const C (&divx)[NV][4], const C (&jx)[2][NV]) {
     using S = typename PA::S_t;
     const Mesh& m = A.m;
     const int lj = l & 3, lk = l >> 2;   // this x-line's (j, k)
     const bool defer = (A.flags & kDeferRK) != 0;
-    C cy[4], cz[4];   // derivative rows of this thread's j (y) and k (z)
+    C cy[4], cz[4];   // derivative rows of this thread's j (y) and k (z); not kWideState: negated
 #pragma unroll
     for (int mm = 0; mm < 4; ++mm) {
-        cy[mm] = A.sc.d[1][lj * 4 + mm];
-        cz[mm] = A.sc.d[2][lk * 4 + mm];
+        cy[mm] = M::kWideState ? A.sc.d[1][lj * 4 + mm] : A.sc.nd[1][lj * 4 + mm];
+        cz[mm] = M::kWideState ? A.sc.d[2][lk * 4 + mm] : A.sc.nd[2][lk * 4 + mm];
     }
 #pragma unroll
     for (int v = 0; v < NV; ++v) {
-        C dy[4], dz[4], jy0[4], jy1[4], jz0[4], jz1[4];
-        const C* dx = divx[v];
-        {
-            C f[4][4];
+        C rt[4], jy0[4], jy1[4], jz0[4], jz1[4];
+        const C* fy = flux_row<M, 1>(sm, v);
+        const C* fz = flux_row<M, 2>(sm, v);
+        if constexpr (M::kWideState) {
+            C dy[4], dz[4];
 #pragma unroll
-            for (int mm = 0; mm < 4; ++mm) ld4s(&sm.g[v][sw(4 * (mm + 4 * lk), swz)], f[mm]);
+            for (int mm = 0; mm < 4; ++mm) {
+                C f[4];
+                ld4s(fy + sw(4 * (mm + 4 * lk), swz), f);
 #pragma unroll
-            for (int i = 0; i < 4; ++i) {
-                C d = cy[0] * f[0][i];
-#pragma unroll
-                for (int mm = 1; mm < 4; ++mm) d = fma(cy[mm], f[mm][i], d);
-                dy[i] = d;
+                for (int i = 0; i < 4; ++i) dy[i] = mm == 0 ? cy[0] * f[i] : fma(cy[mm], f[i], dy[i]);
             }
-        }
-        {
-            C f[4][4];
 #pragma unroll
-            for (int mm = 0; mm < 4; ++mm) ld4s(&sm.g[5 + v][sw(4 * (lj + 4 * mm), swz)], f[mm]);
+            for (int mm = 0; mm < 4; ++mm) {
+                C f[4];
+                ld4s(fz + sw(4 * (lj + 4 * mm), swz), f);
+#pragma unroll
+                for (int i = 0; i < 4; ++i) dz[i] = mm == 0 ? cz[0] * f[i] : fma(cz[mm], f[i], dz[i]);
+            }
 #pragma unroll
             for (int i = 0; i < 4; ++i) {
-                C d = cz[0] * f[0][i];
+                rt[i] = -((divx[v][i] + dy[i]) + dz[i]);
+                if (v == 1) rt[i] += A.forcing;
+            }
+        } else {
 #pragma unroll
-                for (int mm = 1; mm < 4; ++mm) d = fma(cz[mm], f[mm][i], d);
-                dz[i] = d;
+            for (int i = 0; i < 4; ++i) rt[i] = divx[v][i];
+#pragma unroll
+            for (int mm = 0; mm < 4; ++mm) {
+                C f[4];
+                ld4s(fy + sw(4 * (mm + 4 * lk), swz), f);
+#pragma unroll
+                for (int i = 0; i < 4; ++i) rt[i] = fma(cy[mm], f[i], rt[i]);
+            }
+#pragma unroll
+            for (int mm = 0; mm < 4; ++mm) {
+                C f[4];
+                ld4s(fz + sw(4 * (lj + 4 * mm), swz), f);
+#pragma unroll
+                for (int i = 0; i < 4; ++i) rt[i] = fma(cz[mm], f[i], rt[i]);
             }
         }
         ld4s(&sm.j[0][v][4 * lk], jy0);
@@ -789,21 +823,19 @@ __device__ __forceinline__ void stage_a_update(const PA& A, SlotA<P, C>& sm, lon
         ld4s(&sm.j[2][v][4 * lj], jz0);
         ld4s(&sm.j[3][v][4 * lj], jz1);
         const C jx0 = jx[0][v], jx1 = jx[1][v];
-        C rt[4];
 #pragma unroll
         for (int i = 0; i < 4; ++i) {
-            C rvol = -((dx[i] + dy[i]) + dz[i]);
-            if (v == 1) rvol += A.forcing;
+            C r = rt[i];
             if constexpr (sizeof(C) == 8) {
-                if (A.flags & kRoundRhs) rvol = (C)(float)rvol;
+                if (A.flags & kRoundRhs) r = (C)(float)r;
             }
             // lifting -(j_L g_L' + j_R g_R') jac of the six faces (rk.cu:12-25)
-            C r = fma(-jx0, A.sc.gl[0][i], rvol);
-            r = fma(-jx1, A.sc.gr[0][i], r);
-            r = fma(-jy0[i], A.sc.gl[1][lj], r);
-            r = fma(-jy1[i], A.sc.gr[1][lj], r);
-            r = fma(-jz0[i], A.sc.gl[2][lk], r);
-            rt[i] = fma(-jz1[i], A.sc.gr[2][lk], r);
+            r = fma(jx0, A.sc.nl[0][i], r);
+            r = fma(jx1, A.sc.nr[0][i], r);
+            r = fma(jy0[i], A.sc.nl[1][lj], r);
+            r = fma(jy1[i], A.sc.nr[1][lj], r);
+            r = fma(jz0[i], A.sc.nl[2][lk], r);
+            rt[i] = fma(jz1[i], A.sc.nr[2][lk], r);
         }
         S* dst = A.u_out + v * m.npts + ec * NE + 4 * l;
         if (defer) {
@@ -824,7 +856,8 @@ __device__ __forceinline__ void stage_a_update(const PA& A, SlotA<P, C>& sm, lon
 }
 
 // One tile of phase A: EPB elements starting at A.e0 + tile * EPB, LPE
-// threads each. Called by every thread of the block (it synchronises).
+// threads each. Called by whole warps: an element's 16 threads are half of one,
+// so nothing here waits for the block's other warps.
 template <class M, int FLUX, int EPB, bool FEAT = false, class PA>
 __device__ __forceinline__ void stage_a_tile(const PA& A, unsigned char* smem_raw, long long tile) {
     using S = typename PA::S_t;
@@ -857,7 +890,7 @@ __device__ __forceinline__ void stage_a_tile(const PA& A, unsigned char* smem_ra
         }
         st4s(&sm.u[v][sw(4 * l, swz)], qx[v]);
     }
-    __syncthreads();
+    __syncwarp();
     if constexpr (FEAT) stage_a_features(A, sm, ec, l, swz, live, qx);
 
     // ---- P2-P4: face values, gradient, interface fluxes per direction
@@ -866,26 +899,27 @@ __device__ __forceinline__ void stage_a_tile(const PA& A, unsigned char* smem_ra
     C fi[3][NV];      // interface fluxes at the minus faces of this thread's lines
     line_pass<M, FLUX, 0>(A, sm, ec, l, li, live, nxm, nxp, tr[0][0], tr[0][1], jx, fi[0], qx);
     line_pass<M, FLUX, 1>(A, sm, ec, l, li, live, nym, nyp, tr[1][0], tr[1][1], jx, fi[1], qx);
-    __syncthreads();   // the x and y gradients, read by the z faces
+    __syncwarp();   // the x and y gradients, read by the z faces
     line_pass<M, FLUX, 2>(A, sm, ec, l, li, live, nzm, nzp, tr[2][0], tr[2][1], jx, fi[2], qx);
-    __syncthreads();
+    __syncwarp();
 
     // ---- P5: viscous face fluxes of the x and y faces, face records (the z
     // faces are done in the z pass)
     face_grad_pass<M, 0>(A, sm, ec, l, li, false, false, live, tr[0][0], tr[0][1], jx, fi[0]);
     face_grad_pass<M, 1>(A, sm, ec, l, li, nym < 0, nyp < 0, live, tr[1][0], tr[1][1], jx, fi[1]);
-    __syncthreads();
+    __syncwarp();
 
     // ---- P6: pointwise fluxes of the x-line's points (own points only; the
     // point order is rotated by k so the 16 lanes of an element hit distinct
     // banks). F_y, F_z -> smem for the y / z divergences; the x-line's F_x
-    // never leaves the thread: its x-divergence is accumulated here (point i
-    // contributes column i of the x derivative) and kept until P8.
+    // never leaves the thread: its x-divergence (with its sign, on top of the
+    // forcing) is accumulated here (point i contributes column i of the x
+    // derivative) and kept until P8.
     C divx[NV][4];
 #pragma unroll
     for (int v = 0; v < NV; ++v)
 #pragma unroll
-        for (int a = 0; a < 4; ++a) divx[v][a] = (C)0;
+        for (int a = 0; a < 4; ++a) divx[v][a] = !M::kWideState && v == 1 ? A.forcing : (C)0;
     {
         const int lk = l >> 2;
 #pragma unroll 1
@@ -898,29 +932,46 @@ __device__ __forceinline__ void stage_a_tile(const PA& A, unsigned char* smem_ra
             P qp[NV];
 #pragma unroll
             for (int v = 0; v < NV; ++v) qp[v] = sm.u[v][p];
-            C praw;
-            FaceState<C> s = make_face_state<M, C, P>(qp, praw);
-            C F[3][NV];
-            const C mu = viscosity<M>(A.mu, A.suth, s);
-            volume_fluxes<C>(s, praw, g, mu, heat_coeff<M>(mu, A.kappa), F);
+            const FaceState<C> s = make_face_state<M, C, P>(qp);
+            C fx[NV];
+            if constexpr (M::kWideState) {
+                C F[3][NV];
+                const C mu = viscosity<M>(A.mu, A.suth, s);
+                volume_fluxes_wide<C>(s, g, mu, heat_coeff<M>(mu, A.kappa), F);
 #pragma unroll
-            for (int v = 0; v < NV; ++v) {
-                sm.g[v][p] = F[1][v];
-                sm.g[5 + v][p] = F[2][v];
+                for (int v = 0; v < NV; ++v) {
+                    sm.g[v][p] = F[1][v];
+                    sm.g[5 + v][p] = F[2][v];
+                    fx[v] = F[0][v];
+                }
+            } else {
+                const VolumeFluxes<C> F = volume_fluxes<C>(s, g, viscosity<M>(A.mu, A.suth, s));
+                sm.g[kFy1][p] = F.m01;
+                sm.g[kFy2][p] = F.m11;
+                sm.g[kFy3][p] = F.m12;
+                sm.g[kFy4][p] = F.e[1];
+                sm.g[kFz1][p] = F.m02;
+                sm.g[kFz3][p] = F.m22;
+                sm.g[kFz4][p] = F.e[2];
+                fx[0] = s.q[1];
+                fx[1] = F.m00;
+                fx[2] = F.m01;
+                fx[3] = F.m02;
+                fx[4] = F.e[0];
             }
 #pragma unroll
             for (int a = 0; a < 4; ++a) {
-                const C d = A.sc.d[0][a * 4 + i];
+                const C d = M::kWideState ? A.sc.d[0][a * 4 + i] : A.sc.nd[0][a * 4 + i];
 #pragma unroll
-                for (int v = 0; v < NV; ++v) divx[v][a] = fma(d, F[0][v], divx[v][a]);
+                for (int v = 0; v < NV; ++v) divx[v][a] = fma(d, fx[v], divx[v][a]);
             }
         }
     }
-    __syncthreads();
+    __syncwarp();
 
     // ---- P7 + P8: y / z divergences, RHS, lifting, RK combination (or the
     // RHS alone for phase B)
-    if (live) stage_a_update(A, sm, ec, l, swz, divx, jx);
+    if (live) stage_a_update<M>(A, sm, ec, l, swz, divx, jx);
 }
 
 // Blocks per SM the register budget is set for. f32 state arithmetic and
