@@ -279,15 +279,48 @@ __device__ __forceinline__ constexpr bool grad_used(int c) {
     return !((omit >> c) & 1u);
 }
 
-// Shared-memory slot of one element in phase A.
 // ---- shared-memory point layout
-// Points of an element are stored at p ^ (((p >> 3) & 4) | par << 3): the
-// j index is XOR-swizzled with bit 1 of k and with the element's parity
+// 4-byte rows: points of an element are stored at p ^ (((p >> 3) & 4) | par << 3):
+// the j index is XOR-swizzled with bit 1 of k and with the element's parity
 // inside its warp (two elements per warp), and every element slot is a
 // multiple of 32 words plus 16. With these, the three access patterns of a
 // half-warp (16 x-lines as 128-bit vectors, 16 y-lines and 16 z-lines as
 // scalars) hit 32 distinct banks across the whole warp.
-__device__ __forceinline__ int sw(int p, int swz) { return p ^ (((p >> 3) & 4) | swz); }
+// 8-byte rows: an access phase is one element's half-warp of 8-byte words (16
+// bank pairs), or 8 lanes of a 128-bit one. j is XORed with all of k, so that
+// the 16 y-lines, 4 values of i for each k, fall on distinct banks, and the
+// halves of an x-line are swapped for odd k, so that the 128-bit halves of
+// the 8 lines of two k's do. (With the 4-byte swizzle 31% of the wavefronts
+// of the f64 kernel were conflicts; 40^3 f64 step 1.64 -> 1.60 ms, 96^3 mixed
+// 15.6 -> 15.0.)
+template <class T>
+__device__ __forceinline__ int sw(int p, int swz) {
+    if constexpr (sizeof(T) == 4)
+        return p ^ (((p >> 3) & 4) | swz);
+    else
+        return p ^ ((p >> 2) & 12) ^ ((p >> 3) & 2);
+}
+
+// the x-line stored at offset x (sw of its first point) of a row
+template <class T>
+__device__ __forceinline__ void ld_xline(const T* row, int x, T* q) {
+    if constexpr (sizeof(T) == 4) {
+        ld4s(row + x, q);
+    } else {
+        const double2 a = *reinterpret_cast<const double2*>(row + x), b = *reinterpret_cast<const double2*>(row + (x ^ 2));
+        q[0] = a.x; q[1] = a.y; q[2] = b.x; q[3] = b.y;
+    }
+}
+
+template <class T>
+__device__ __forceinline__ void st_xline(T* row, int x, const T* q) {
+    if constexpr (sizeof(T) == 4) {
+        st4s(row + x, q);
+    } else {
+        *reinterpret_cast<double2*>(row + x) = make_double2(q[0], q[1]);
+        *reinterpret_cast<double2*>(row + (x ^ 2)) = make_double2(q[2], q[3]);
+    }
+}
 
 template <class P, class C>
 struct SlotBytes {
@@ -349,8 +382,8 @@ __device__ __forceinline__ void stage_a_features(const PA& A, SlotA<P, C>& sm, l
         float ly[4][4], lz[4][4];   // the x-lines (m, k) and (j, m), m = 0..3
 #pragma unroll
         for (int m = 0; m < 4; ++m) {
-            ld4s(&sm.u[v][sw(4 * (m + 4 * k), swz)], ly[m]);
-            ld4s(&sm.u[v][sw(4 * (j + 4 * m), swz)], lz[m]);
+            ld_xline(sm.u[v], sw<P>(4 * (m + 4 * k), swz), ly[m]);
+            ld_xline(sm.u[v], sw<P>(4 * (j + 4 * m), swz), lz[m]);
         }
 #pragma unroll
         for (int i = 0; i < 4; ++i) {
@@ -443,45 +476,67 @@ __device__ __forceinline__ void plus_face(const FaceState<C>& so, bool wall, C* 
 }
 
 // Swizzled row offsets of the three lines of thread l, computed once per
-// tile: x-line start, the four y-line points and the two z-line bases
-// (points mm < 2 and mm >= 2, + 16 mm).
+// tile: x-line start, the four y-line points and the z-line points (4-byte
+// rows: the bases of points mm < 2 and mm >= 2, + 16 mm).
+template <class T>
 struct LineIdx {
     int x;
     int y[4];
-    int z[2];
+    int z[sizeof(T) == 4 ? 2 : 4];
 };
 
-__device__ __forceinline__ LineIdx line_idx(int l, int swz) {
-    LineIdx li;
-    li.x = sw(4 * l, swz);
+template <class T>
+__device__ __forceinline__ LineIdx<T> line_idx(int l, int swz) {
+    LineIdx<T> li;
+    li.x = sw<T>(4 * l, swz);
 #pragma unroll
-    for (int mm = 0; mm < 4; ++mm) li.y[mm] = sw(line_pt<1>(l, mm), swz);
-    li.z[0] = sw(line_pt<2>(l, 0), swz);
-    li.z[1] = sw(line_pt<2>(l, 2), swz) - 32;
+    for (int mm = 0; mm < 4; ++mm) li.y[mm] = sw<T>(line_pt<1>(l, mm), swz);
+    if constexpr (sizeof(T) == 4) {
+        li.z[0] = sw<T>(line_pt<2>(l, 0), swz);
+        li.z[1] = sw<T>(line_pt<2>(l, 2), swz) - 32;
+    } else {
+#pragma unroll
+        for (int mm = 0; mm < 4; ++mm) li.z[mm] = sw<T>(line_pt<2>(l, mm), swz);
+    }
     return li;
 }
 
-template <int D>
-__device__ __forceinline__ int line_off(const LineIdx& li, int mm) {
+template <int D, class T>
+__device__ __forceinline__ int line_off(const LineIdx<T>& li, int mm) {
     if constexpr (D == 1) return li.y[mm];
-    else return li.z[mm >> 1] + 16 * mm;
+    else if constexpr (sizeof(T) == 4) return li.z[mm >> 1] + 16 * mm;
+    else return li.z[mm];
 }
 
+// the offsets in rows of the state type and of the flux type
+template <class P, class C>
+struct LineSet {
+    LineIdx<P> p;
+    LineIdx<C> c;
+    template <class T>
+    __device__ __forceinline__ const auto& of() const {
+        if constexpr (sizeof(T) == sizeof(P)) return p;
+        else return c;
+    }
+};
+
 // load / store the 4 samples of the thread's direction-D line of a swizzled row
-template <int D, class T>
-__device__ __forceinline__ void row_line_load(const T* row, const LineIdx& li, T* w) {
+template <int D, class T, class L>
+__device__ __forceinline__ void row_line_load(const T* row, const L& ls, T* w) {
+    const auto& li = ls.template of<T>();
     if constexpr (D == 0) {
-        ld4s(row + li.x, w);
+        ld_xline(row, li.x, w);
     } else {
 #pragma unroll
         for (int mm = 0; mm < 4; ++mm) w[mm] = row[line_off<D>(li, mm)];
     }
 }
 
-template <int D, class T>
-__device__ __forceinline__ void row_line_store(T* row, const LineIdx& li, const T* w) {
+template <int D, class T, class L>
+__device__ __forceinline__ void row_line_store(T* row, const L& ls, const T* w) {
+    const auto& li = ls.template of<T>();
     if constexpr (D == 0) {
-        st4s(row + li.x, w);
+        st_xline(row, li.x, w);
     } else {
 #pragma unroll
         for (int mm = 0; mm < 4; ++mm) row[line_off<D>(li, mm)] = w[mm];
@@ -532,7 +587,7 @@ __device__ __forceinline__ void viscous_face(const PA& A, SlotA<P, C>& sm, long 
 // part (P5 for z): its normal gradient components are traced from registers
 // and the z-face corrections are stored once, complete.
 template <class M, int FLUX, int D, class PA, class P = typename PA::P_t, class C = typename PA::C_t>
-__device__ __forceinline__ void line_pass(const PA& A, SlotA<P, C>& sm, long long e, int l, const LineIdx& li,
+__device__ __forceinline__ void line_pass(const PA& A, SlotA<P, C>& sm, long long e, int l, const LineSet<P, C>& li,
                                           bool live, const long long nb0, const long long nb1, P* oL, P* oR,
                                           C (&jx)[2][NV], C* fi, const P (&qx)[NV][4]) {
     using S = typename PA::S_t;
@@ -691,7 +746,7 @@ __device__ __forceinline__ C ref_y_slice(const C* w, const CC& c) {
 // flux at both faces of the line.
 template <class M, int D, class PA, class P = typename PA::P_t, class C = typename PA::C_t>
 __device__ __forceinline__ void face_grad_pass(const PA& A, SlotA<P, C>& sm, long long e, int l,
-                                               const LineIdx& li, bool wall0, bool wall1, bool live, const P* tL,
+                                               const LineSet<P, C>& li, bool wall0, bool wall1, bool live, const P* tL,
                                                const P* tR, C (&jx)[2][NV], const C* fi) {
     if (wall0 && wall1) return;
     C gL[15], gR[15];
@@ -784,14 +839,14 @@ __device__ __forceinline__ void stage_a_update(const PA& A, SlotA<P, C>& sm, lon
 #pragma unroll
             for (int mm = 0; mm < 4; ++mm) {
                 C f[4];
-                ld4s(fy + sw(4 * (mm + 4 * lk), swz), f);
+                ld_xline(fy, sw<C>(4 * (mm + 4 * lk), swz), f);
 #pragma unroll
                 for (int i = 0; i < 4; ++i) dy[i] = mm == 0 ? cy[0] * f[i] : fma(cy[mm], f[i], dy[i]);
             }
 #pragma unroll
             for (int mm = 0; mm < 4; ++mm) {
                 C f[4];
-                ld4s(fz + sw(4 * (lj + 4 * mm), swz), f);
+                ld_xline(fz, sw<C>(4 * (lj + 4 * mm), swz), f);
 #pragma unroll
                 for (int i = 0; i < 4; ++i) dz[i] = mm == 0 ? cz[0] * f[i] : fma(cz[mm], f[i], dz[i]);
             }
@@ -806,14 +861,14 @@ __device__ __forceinline__ void stage_a_update(const PA& A, SlotA<P, C>& sm, lon
 #pragma unroll
             for (int mm = 0; mm < 4; ++mm) {
                 C f[4];
-                ld4s(fy + sw(4 * (mm + 4 * lk), swz), f);
+                ld_xline(fy, sw<C>(4 * (mm + 4 * lk), swz), f);
 #pragma unroll
                 for (int i = 0; i < 4; ++i) rt[i] = fma(cy[mm], f[i], rt[i]);
             }
 #pragma unroll
             for (int mm = 0; mm < 4; ++mm) {
                 C f[4];
-                ld4s(fz + sw(4 * (lj + 4 * mm), swz), f);
+                ld_xline(fz, sw<C>(4 * (lj + 4 * mm), swz), f);
 #pragma unroll
                 for (int i = 0; i < 4; ++i) rt[i] = fma(cz[mm], f[i], rt[i]);
             }
@@ -866,7 +921,7 @@ __device__ __forceinline__ void stage_a_tile(const PA& A, unsigned char* smem_ra
     const int l = threadIdx.x & (LPE - 1);
     const int es = threadIdx.x / LPE;
     const int swz = (es & 1) << 3;
-    const LineIdx li = line_idx(l, swz);
+    const LineSet<P, C> li{line_idx<P>(l, swz), line_idx<C>(l, swz)};
     SlotA<P, C>& sm = reinterpret_cast<SlotA<P, C>*>(smem_raw)[es];
     const long long e = A.e0 + tile * EPB + es;
     const bool live = e < A.e1;
@@ -888,7 +943,7 @@ __device__ __forceinline__ void stage_a_tile(const PA& A, unsigned char* smem_ra
 #pragma unroll
             for (int a = 0; a < 4; ++a) qx[v][a] = (P)1.0;
         }
-        st4s(&sm.u[v][sw(4 * l, swz)], qx[v]);
+        st_xline(sm.u[v], li.p.x, qx[v]);
     }
     __syncwarp();
     if constexpr (FEAT) stage_a_features(A, sm, ec, l, swz, live, qx);
@@ -925,13 +980,13 @@ __device__ __forceinline__ void stage_a_tile(const PA& A, unsigned char* smem_ra
 #pragma unroll 1
         for (int it = 0; it < 4; ++it) {
             const int i = (it + lk) & 3;
-            const int p = sw(4 * l + i, swz);
+            const int p = sw<C>(4 * l + i, swz), pp = sw<P>(4 * l + i, swz);
             C g[15];
 #pragma unroll
             for (int c = 0; c < 15; ++c) g[c] = sm.g[c][p];
             P qp[NV];
 #pragma unroll
-            for (int v = 0; v < NV; ++v) qp[v] = sm.u[v][p];
+            for (int v = 0; v < NV; ++v) qp[v] = sm.u[v][pp];
             const FaceState<C> s = make_face_state<M, C, P>(qp);
             C fx[NV];
             if constexpr (M::kWideState) {
