@@ -46,7 +46,7 @@ namespace {
 using od::LPE;
 using od::NE;
 using od::NF;
-using od::SlotA;
+using Slot = od::SlotFor<od::MathFast, float, float>;   // one element of phase A
 // FR tables of every box (identical) in constant memory; the stage code reads
 // them through these proxies with compile-time offsets, as it reads kernel
 // parameters in the single-box kernels.
@@ -227,7 +227,7 @@ __global__ void __launch_bounds__(LPE * EPB, 16 / EPB * 2) ensemble_stage_kernel
     {
         const long long total = start_b[nbox];
         StageB* Bs = reinterpret_cast<StageB*>(smem_raw);
-        const bool in_smem = !CP && (size_t)nbox * sizeof(StageB) <= sizeof(SlotA<float, float>) * EPB;
+        const bool in_smem = !CP && (size_t)nbox * sizeof(StageB) <= sizeof(Slot) * EPB;
         if (in_smem) {
             for (int b = 0; b < nbox; ++b) block_copy(&Bs[b], &boxes[b].B);
             __syncthreads();
@@ -378,7 +378,7 @@ void* pick_kernel(bool fast, int epb, bool cp) {
     return epb == 2 ? kernel_ptr<od::MathIeee, 2>(cp) : kernel_ptr<od::MathIeee, 4>(cp);
 }
 
-size_t dyn_smem(int epb) { return sizeof(SlotA<float, float>) * (size_t)epb; }
+size_t dyn_smem(int epb) { return sizeof(Slot) * (size_t)epb; }
 
 }  // namespace
 

@@ -34,7 +34,7 @@ template <class S, class P, class C, class M, int FLUX, int EPB>
 cudaError_t launch_a(const StageAParams<S, P, C>& A, long long nelem, cudaStream_t s, bool feat = false) {
     const unsigned grid = (unsigned)((nelem + EPB - 1) / EPB);
     if (grid == 0) return cudaSuccess;
-    const size_t smem = sizeof(SlotA<P, C>) * EPB;
+    const size_t smem = sizeof(SlotFor<M, P, C>) * EPB;
     if constexpr (has_feat_variant<S, P, C, M>() && EPB == 4) {
         if (feat) {
             stage_a_kernel<S, P, C, M, FLUX, EPB, true><<<grid, LPE * EPB, smem, s>>>(A);
@@ -178,13 +178,13 @@ template <class S, class P, class C, class M, int FLUX>
 cudaError_t prepare_flux() {
     cudaError_t e = cudaFuncSetAttribute(stage_a_kernel<S, P, C, M, FLUX, 2>,
                                          cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         (int)(sizeof(SlotA<P, C>) * 2));
+                                         (int)(sizeof(SlotFor<M, P, C>) * 2));
     if (e != cudaSuccess) return e;
     e = cudaFuncSetAttribute(stage_a_kernel<S, P, C, WithSutherland<M>, FLUX, 4>,
-                             cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(sizeof(SlotA<P, C>) * 4));
+                             cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(sizeof(SlotFor<M, P, C>) * 4));
     if (e != cudaSuccess) return e;
     return cudaFuncSetAttribute(stage_a_kernel<S, P, C, M, FLUX, 4>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                (int)(sizeof(SlotA<P, C>) * 4));
+                                (int)(sizeof(SlotFor<M, P, C>) * 4));
 }
 
 template <class S, class P, class C, class M>

@@ -322,22 +322,42 @@ __device__ __forceinline__ void st_xline(T* row, int x, const T* q) {
     }
 }
 
-template <class P, class C>
+// Whether every face correction of a line stays in its thread's registers
+// (the all-f32 kernels): the update then works on the thread's own y- and
+// z-lines, one row line in and one out per variable, where the update of a
+// whole x-line loads the four x-lines of its k-plane and of its j-column and
+// the corrections of four lines (960 bytes a thread, a third of the kernel's
+// shared-memory traffic). f64 needs the registers.
+template <class M, class P, class C>
+constexpr bool kLineUpdate = !M::kWideState && sizeof(P) == 4 && sizeof(C) == 4;
+
+template <class P, class C, bool J>
 struct SlotBytes {
-    static constexpr int base = 15 * NE * (int)sizeof(C) + NV * NE * (int)sizeof(P) + 4 * NV * NF * (int)sizeof(C);
+    static constexpr int base =
+        15 * NE * (int)sizeof(C) + NV * NE * (int)sizeof(P) + (J ? 4 * NV * NF * (int)sizeof(C) : 0);
     static constexpr int words = base / 4;
     static constexpr int pad_words = ((16 - words % 32) + 32) % 32 == 0 ? 32 : ((16 - words % 32) + 32) % 32;
 };
 
-// Shared-memory slot of one element in phase A.
-template <class P, class C>
-struct alignas(16) SlotA {
-    C g[15][NE];          // gradient; P6: F_y rows 0-4, F_z rows 5-9
-    P u[NV][NE];          // state
-    C j[4][NV][NF];       // y / z face corrections without -1/2 Fv_nbr [face - 2][var][face pt]; the x faces of
-                          // a line belong to its own thread and stay in registers
-    float pad[SlotBytes<P, C>::pad_words];
+// y / z face corrections without -1/2 Fv_nbr [face - 2][var][face pt]; the x
+// faces of a line belong to its own thread and stay in registers
+template <class C, bool J>
+struct SlotJ {
+    C j[4][NV][NF];
 };
+template <class C>
+struct SlotJ<C, false> {};
+
+// Shared-memory slot of one element in phase A.
+template <class P, class C, bool J>
+struct alignas(16) SlotA : SlotJ<C, J> {
+    C g[15][NE];          // gradient; from P6: fluxes (and partial updates) in the first rows
+    P u[NV][NE];          // state
+    float pad[SlotBytes<P, C, J>::pad_words];
+};
+
+template <class M, class P, class C>
+using SlotFor = SlotA<P, C, !kLineUpdate<M, P, C>>;
 
 template <class S, class P, class C>
 struct StageAParams {
@@ -371,8 +391,8 @@ struct StageAParams {
 // x-line, y / z derivatives from the x-lines of its k-plane / j-column),
 // staged as bf16 in the gradient rows (not written before P2) and stored in
 // the fused inference kernel's tile layout as 16-byte chunks.
-template <class PA, class P = typename PA::P_t, class C = typename PA::C_t>
-__device__ __forceinline__ void stage_a_features(const PA& A, SlotA<P, C>& sm, long long e, int l, int swz,
+template <class PA, class Slot, class P = typename PA::P_t, class C = typename PA::C_t>
+__device__ __forceinline__ void stage_a_features(const PA& A, Slot& sm, long long e, int l, int swz,
                                                  bool live, const P (&qx)[NV][4]) {
     const StageFeatures& fp = A.feat;
     const int j = l & 3, k = l >> 2;
@@ -549,8 +569,8 @@ __device__ __forceinline__ void row_line_store(T* row, const L& ls, const T* w) 
 // plus face.
 // REG: the face's correction j is in registers (jreg), else in shared memory.
 // s: the face state (make_face_state of the face values).
-template <class M, int D, bool REG, class PA, class P = typename PA::P_t, class C = typename PA::C_t>
-__device__ __forceinline__ void viscous_face(const PA& A, SlotA<P, C>& sm, long long e, int l, int side,
+template <class M, int D, bool REG, class PA, class Slot, class P = typename PA::P_t, class C = typename PA::C_t>
+__device__ __forceinline__ void viscous_face(const PA& A, Slot& sm, long long e, int l, int side,
                                              const FaceState<C>& s, const C* gt, bool live, C* jreg,
                                              const C* fi) {
     const int f = 2 * D + side;
@@ -581,15 +601,16 @@ __device__ __forceinline__ void viscous_face(const PA& A, SlotA<P, C>& sm, long 
 }
 
 // P2-P4: one direction of the gradient / face-value pass for line l.
+// jd: the corrections at the line's two faces, where they stay in registers.
 // qx: the thread's own x-line as P1 loaded it (used by the x pass instead of
 // reading it back from shared memory). The z pass (the last one, run after
 // the x and y gradients are in shared memory) also does the z faces' viscous
 // part (P5 for z): its normal gradient components are traced from registers
 // and the z-face corrections are stored once, complete.
-template <class M, int FLUX, int D, class PA, class P = typename PA::P_t, class C = typename PA::C_t>
-__device__ __forceinline__ void line_pass(const PA& A, SlotA<P, C>& sm, long long e, int l, const LineSet<P, C>& li,
+template <class M, int FLUX, int D, class PA, class Slot, class P = typename PA::P_t, class C = typename PA::C_t>
+__device__ __forceinline__ void line_pass(const PA& A, Slot& sm, long long e, int l, const LineSet<P, C>& li,
                                           bool live, const long long nb0, const long long nb1, P* oL, P* oR,
-                                          C (&jx)[2][NV], C* fi, const P (&qx)[NV][4]) {
+                                          C (&jd)[2][NV], C* fi, const P (&qx)[NV][4]) {
     using S = typename PA::S_t;
     const Mesh& m = A.m;
     P q[NV][4];
@@ -722,9 +743,9 @@ __device__ __forceinline__ void line_pass(const PA& A, SlotA<P, C>& sm, long lon
     }
 #pragma unroll
     for (int v = 0; v < NV; ++v) {
-        if constexpr (D == 0) {
-            jx[0][v] = j0[v];
-            jx[1][v] = j1[v];
+        if constexpr (D == 0 || kLineUpdate<M, P, C>) {
+            jd[0][v] = j0[v];
+            jd[1][v] = j1[v];
         } else {
             sm.j[2 * D - 2][v][l] = j0[v];
             sm.j[2 * D - 1][v][l] = j1[v];
@@ -744,10 +765,10 @@ __device__ __forceinline__ C ref_y_slice(const C* w, const CC& c) {
 
 // P5: face values and face gradient along the D-line of thread l, viscous
 // flux at both faces of the line.
-template <class M, int D, class PA, class P = typename PA::P_t, class C = typename PA::C_t>
-__device__ __forceinline__ void face_grad_pass(const PA& A, SlotA<P, C>& sm, long long e, int l,
+template <class M, int D, class PA, class Slot, class P = typename PA::P_t, class C = typename PA::C_t>
+__device__ __forceinline__ void face_grad_pass(const PA& A, Slot& sm, long long e, int l,
                                                const LineSet<P, C>& li, bool wall0, bool wall1, bool live, const P* tL,
-                                               const P* tR, C (&jx)[2][NV], const C* fi) {
+                                               const P* tR, C (&jd)[2][NV], const C* fi) {
     if (wall0 && wall1) return;
     C gL[15], gR[15];
     const bool ref_y = D == 1 && sizeof(C) == 8 && (A.flags & kRefYSlice);
@@ -782,11 +803,11 @@ __device__ __forceinline__ void face_grad_pass(const PA& A, SlotA<P, C>& sm, lon
     }
     if (!wall0) {
         const FaceState<C> st = make_face_state<M, C, P>(qL);
-        viscous_face<M, D, D == 0>(A, sm, e, l, 0, st, gL, live, jx[0], fi);
+        viscous_face<M, D, D == 0 || kLineUpdate<M, P, C>>(A, sm, e, l, 0, st, gL, live, jd[0], fi);
     }
     if (!wall1) {
         const FaceState<C> st = make_face_state<M, C, P>(qR);
-        viscous_face<M, D, D == 0>(A, sm, e, l, 1, st, gR, live, jx[1], fi);
+        viscous_face<M, D, D == 0 || kLineUpdate<M, P, C>>(A, sm, e, l, 1, st, gR, live, jd[1], fi);
     }
 }
 
@@ -795,15 +816,39 @@ __device__ __forceinline__ void face_grad_pass(const PA& A, SlotA<P, C>& sm, lon
 // state (kWideState: all ten fluxes in rows 0-9).
 constexpr int kFy1 = 0, kFy2 = 1, kFy3 = 2, kFy4 = 3, kFz1 = 4, kFz2 = kFy3, kFz3 = 5, kFz4 = 6;
 
-template <class M, int D, class P, class C>
-__device__ __forceinline__ const C* flux_row(const SlotA<P, C>& sm, int v) {
+template <class M, int D, class Slot>
+__device__ __forceinline__ const auto* flux_row(const Slot& sm, int v) {
     if constexpr (M::kWideState) {
-        return sm.g[(D == 1 ? 0 : 5) + v];
+        return &sm.g[(D == 1 ? 0 : 5) + v][0];
     } else if constexpr (D == 1) {
-        return v == 0 ? sm.u[2] : sm.g[v == 1 ? kFy1 : v == 2 ? kFy2 : v == 3 ? kFy3 : kFy4];
+        return v == 0 ? &sm.u[2][0] : &sm.g[v == 1 ? kFy1 : v == 2 ? kFy2 : v == 3 ? kFy3 : kFy4][0];
     } else {
-        return v == 0 ? sm.u[3] : sm.g[v == 1 ? kFz1 : v == 2 ? kFz2 : v == 3 ? kFz3 : kFz4];
+        return v == 0 ? &sm.u[3][0] : &sm.g[v == 1 ? kFz1 : v == 2 ? kFz2 : v == 3 ? kFz3 : kFz4][0];
     }
+}
+
+// RK combination a*u0 + b*u + c*R of variable v on the x-line, or (deferred
+// RK) the unrounded R for phase B.
+template <class PA, class P = typename PA::P_t, class C = typename PA::C_t>
+__device__ __forceinline__ void store_update(const PA& A, long long ec, int l, int v, const C (&rt)[4]) {
+    using S = typename PA::S_t;
+    const Mesh& m = A.m;
+    const bool defer = (A.flags & kDeferRK) != 0;
+    S* dst = A.u_out + v * m.npts + ec * NE + 4 * l;
+    if (defer) {
+        stg4<S, C>(dst, rt);
+        return;
+    }
+    P un[4], u0v[4], out[4];
+    ldg4<S, P>(A.u_in + v * m.npts + ec * NE + 4 * l, un);
+    if (A.flags & kHasU0) ldc4<S, P>(A.u0 + v * m.npts + ec * NE + 4 * l, u0v);
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+        P o = A.rb * un[i] + A.rc * (P)rt[i];
+        if (A.flags & kHasU0) o = A.ra * u0v[i] + A.rb * un[i] + A.rc * (P)rt[i];
+        out[i] = o;
+    }
+    stg4<S, P>(dst, out);
 }
 
 // P7 + P8 of phase A for one live element: the y / z divergences of the
@@ -816,13 +861,10 @@ __device__ __forceinline__ const C* flux_row(const SlotA<P, C>& sm, int v) {
 // of the same plane / column load the same line: broadcasts), so no pass
 // along y and z lines and no barrier before the update. Operation order per
 // point as a derivative along the line: D[a][0] F_0, then FMAs for m = 1..3.
-template <class M, class PA, class P = typename PA::P_t, class C = typename PA::C_t>
-__device__ __forceinline__ void stage_a_update(const PA& A, SlotA<P, C>& sm, long long ec, int l, int swz,
+template <class M, class PA, class Slot, class P = typename PA::P_t, class C = typename PA::C_t>
+__device__ __forceinline__ void stage_a_update(const PA& A, Slot& sm, long long ec, int l, int swz,
                                                const C (&divx)[NV][4], const C (&jx)[2][NV]) {
-    using S = typename PA::S_t;
-    const Mesh& m = A.m;
     const int lj = l & 3, lk = l >> 2;   // this x-line's (j, k)
-    const bool defer = (A.flags & kDeferRK) != 0;
     C cy[4], cz[4];   // derivative rows of this thread's j (y) and k (z); not kWideState: negated
 #pragma unroll
     for (int mm = 0; mm < 4; ++mm) {
@@ -892,21 +934,62 @@ __device__ __forceinline__ void stage_a_update(const PA& A, SlotA<P, C>& sm, lon
             r = fma(jz0[i], A.sc.nl[2][lk], r);
             rt[i] = fma(jz1[i], A.sc.nr[2][lk], r);
         }
-        S* dst = A.u_out + v * m.npts + ec * NE + 4 * l;
-        if (defer) {
-            stg4<S, C>(dst, rt);
-            continue;
-        }
-        P un[4], u0v[4], out[4];
-        ldg4<S, P>(A.u_in + v * m.npts + ec * NE + 4 * l, un);
-        if (A.flags & kHasU0) ldc4<S, P>(A.u0 + v * m.npts + ec * NE + 4 * l, u0v);
+        store_update(A, ec, l, v, rt);
+    }
+}
+
+// P7 + P8 with the face corrections in registers (kLineUpdate): the thread's
+// y-line takes the y divergence and the lifting of its two faces into rows
+// kR.., its z-line adds the z terms, and the x-line adds divx and the x lifting.
+// One line of four values in and out of shared memory per variable and
+// direction. Called by whole warps.
+constexpr int kR = 7;   // first row of the partial updates (rows 0-6: the fluxes)
+
+template <class M, class PA, class Slot, class P = typename PA::P_t, class C = typename PA::C_t>
+__device__ __forceinline__ void stage_a_update_lines(const PA& A, Slot& sm, long long ec, int l,
+                                                     const LineSet<P, C>& li, bool live, const C (&divx)[NV][4],
+                                                     const C (&jx)[2][NV], const C (&jy)[2][NV],
+                                                     const C (&jz)[2][NV]) {
 #pragma unroll
-        for (int i = 0; i < 4; ++i) {
-            P o = A.rb * un[i] + A.rc * (P)rt[i];
-            if (A.flags & kHasU0) o = A.ra * u0v[i] + A.rb * un[i] + A.rc * (P)rt[i];
-            out[i] = o;
+    for (int v = 0; v < NV; ++v) {
+        C f[4], r[4];
+        row_line_load<1>(flux_row<M, 1>(sm, v), li, f);
+#pragma unroll
+        for (int a = 0; a < 4; ++a) {
+            r[a] = jy[0][v] * A.sc.nl[1][a];
+            r[a] = fma(jy[1][v], A.sc.nr[1][a], r[a]);
+#pragma unroll
+            for (int mm = 0; mm < 4; ++mm) r[a] = fma(A.sc.nd[1][a * 4 + mm], f[mm], r[a]);
         }
-        stg4<S, P>(dst, out);
+        row_line_store<1>(sm.g[kR + v], li, r);
+    }
+    __syncwarp();
+#pragma unroll
+    for (int v = 0; v < NV; ++v) {
+        C f[4], r[4];
+        row_line_load<2>(flux_row<M, 2>(sm, v), li, f);
+        row_line_load<2>(sm.g[kR + v], li, r);
+#pragma unroll
+        for (int a = 0; a < 4; ++a) {
+            r[a] = fma(jz[0][v], A.sc.nl[2][a], r[a]);
+            r[a] = fma(jz[1][v], A.sc.nr[2][a], r[a]);
+#pragma unroll
+            for (int mm = 0; mm < 4; ++mm) r[a] = fma(A.sc.nd[2][a * 4 + mm], f[mm], r[a]);
+        }
+        row_line_store<2>(sm.g[kR + v], li, r);
+    }
+    __syncwarp();
+#pragma unroll
+    for (int v = 0; v < NV; ++v) {
+        C r[4];
+        row_line_load<0>(sm.g[kR + v], li, r);
+#pragma unroll
+        for (int a = 0; a < 4; ++a) {
+            r[a] += divx[v][a];
+            r[a] = fma(jx[0][v], A.sc.nl[0][a], r[a]);
+            r[a] = fma(jx[1][v], A.sc.nr[0][a], r[a]);
+        }
+        if (live) store_update(A, ec, l, v, r);
     }
 }
 
@@ -922,7 +1005,7 @@ __device__ __forceinline__ void stage_a_tile(const PA& A, unsigned char* smem_ra
     const int es = threadIdx.x / LPE;
     const int swz = (es & 1) << 3;
     const LineSet<P, C> li{line_idx<P>(l, swz), line_idx<C>(l, swz)};
-    SlotA<P, C>& sm = reinterpret_cast<SlotA<P, C>*>(smem_raw)[es];
+    SlotFor<M, P, C>& sm = reinterpret_cast<SlotFor<M, P, C>*>(smem_raw)[es];
     const long long e = A.e0 + tile * EPB + es;
     const bool live = e < A.e1;
     const long long ec = live ? e : 0;
@@ -951,17 +1034,18 @@ __device__ __forceinline__ void stage_a_tile(const PA& A, unsigned char* smem_ra
     // ---- P2-P4: face values, gradient, interface fluxes per direction
     P tr[3][2][NV];   // own face values of this thread's lines (kept only for f32 state arithmetic)
     C jx[2][NV];      // this x-line's x-face corrections
+    C jy[2][NV], jz[2][NV];   // kLineUpdate: the y- and z-line's
     C fi[3][NV];      // interface fluxes at the minus faces of this thread's lines
     line_pass<M, FLUX, 0>(A, sm, ec, l, li, live, nxm, nxp, tr[0][0], tr[0][1], jx, fi[0], qx);
-    line_pass<M, FLUX, 1>(A, sm, ec, l, li, live, nym, nyp, tr[1][0], tr[1][1], jx, fi[1], qx);
+    line_pass<M, FLUX, 1>(A, sm, ec, l, li, live, nym, nyp, tr[1][0], tr[1][1], jy, fi[1], qx);
     __syncwarp();   // the x and y gradients, read by the z faces
-    line_pass<M, FLUX, 2>(A, sm, ec, l, li, live, nzm, nzp, tr[2][0], tr[2][1], jx, fi[2], qx);
+    line_pass<M, FLUX, 2>(A, sm, ec, l, li, live, nzm, nzp, tr[2][0], tr[2][1], jz, fi[2], qx);
     __syncwarp();
 
     // ---- P5: viscous face fluxes of the x and y faces, face records (the z
     // faces are done in the z pass)
     face_grad_pass<M, 0>(A, sm, ec, l, li, false, false, live, tr[0][0], tr[0][1], jx, fi[0]);
-    face_grad_pass<M, 1>(A, sm, ec, l, li, nym < 0, nyp < 0, live, tr[1][0], tr[1][1], jx, fi[1]);
+    face_grad_pass<M, 1>(A, sm, ec, l, li, nym < 0, nyp < 0, live, tr[1][0], tr[1][1], jy, fi[1]);
     __syncwarp();
 
     // ---- P6: pointwise fluxes of the x-line's points (own points only; the
@@ -1026,7 +1110,10 @@ __device__ __forceinline__ void stage_a_tile(const PA& A, unsigned char* smem_ra
 
     // ---- P7 + P8: y / z divergences, RHS, lifting, RK combination (or the
     // RHS alone for phase B)
-    if (live) stage_a_update<M>(A, sm, ec, l, swz, divx, jx);
+    if constexpr (kLineUpdate<M, P, C>)
+        stage_a_update_lines<M>(A, sm, ec, l, li, live, divx, jx, jy, jz);
+    else if (live)
+        stage_a_update<M>(A, sm, ec, l, swz, divx, jx);
 }
 
 // Blocks per SM the register budget is set for. f32 state arithmetic and
