@@ -261,6 +261,77 @@ __device__ __forceinline__ VolumeFluxes<C> volume_fluxes(const FaceState<C>& s, 
     return f;
 }
 
+// The same at two points at once in packed f32 arithmetic (FFMA2: two lanes an
+// instruction; the kernels are bound by instruction issue, not by the FP32
+// pipe). Every multiply-add is explicit.
+struct F2 {
+    float2 v;
+    __device__ __forceinline__ F2() {}
+    __device__ __forceinline__ F2(float a) : v{a, a} {}
+    __device__ __forceinline__ F2(float a, float b) : v{a, b} {}
+    __device__ __forceinline__ F2(float2 a) : v(a) {}
+};
+__device__ __forceinline__ F2 operator*(F2 a, F2 b) { return __fmul2_rn(a.v, b.v); }
+__device__ __forceinline__ F2 operator+(F2 a, F2 b) { return __fadd2_rn(a.v, b.v); }
+__device__ __forceinline__ F2 fma2(F2 a, F2 b, F2 c) { return __ffma2_rn(a.v, b.v, c.v); }
+__device__ __forceinline__ F2 neg2(F2 a) { return F2(-a.v.x, -a.v.y); }
+
+struct VolumeFluxes2 {
+    F2 m00, m11, m22, m01, m02, m12;
+    F2 e[3];
+};
+
+// q(v), g(c): the conserved variables and gradient components of the two points
+template <class M, class QF, class GF>
+__device__ __forceinline__ VolumeFluxes2 volume_fluxes2(QF q, GF g, float mu0, float suth) {
+    const F2 q0 = q(0), q1 = q(1), q2 = q(2), q3 = q(3), q4 = q(4);
+    const F2 ir(M::rcp(q0.v.x), M::rcp(q0.v.y));
+    const F2 nir = neg2(ir);
+    const F2 u = q1 * ir, v = q2 * ir, x = q3 * ir;
+    const F2 nu = q1 * nir, nv = q2 * nir, nx = q3 * nir;
+    const F2 s2 = fma2(q3, x, fma2(q2, v, q1 * u));   // 2 ke
+    const F2 ein = fma2(s2, F2(-0.5f), q4);
+    const F2 pr = ein * F2(Gas<float>::gm1());
+    const F2 p(clamp_p<float>(pr.v.x), clamp_p<float>(pr.v.y));
+    F2 mu(mu0);
+    if constexpr (M::kSutherland) {
+        FaceState<float> a, b;
+        a.p = p.v.x; a.ir = ir.v.x;
+        b.p = p.v.y; b.ir = ir.v.y;
+        mu = F2(viscosity<M>(mu0, suth, a), viscosity<M>(mu0, suth, b));
+    }
+    const F2 nmi = mu * nir;                       // -mu / rho
+    const F2 ce = fma2(s2, F2(0.5f), neg2(ein)) * ir;   // (ke - ein) / rho
+    const F2 h = q4 + p;
+    VolumeFluxes2 f;
+    const F2 r0 = g(0), r1 = g(1), r2 = g(2);      // gradient of rho
+    const F2 a00 = g(3), a10 = g(6), a20 = g(9);   // d/dx of the momenta
+    const F2 a01 = g(4), a11 = g(7), a21 = g(10);
+    const F2 a02 = g(5), a12 = g(8), a22 = g(11);
+    const F2 w00 = fma2(nu, r0, a00), w11 = fma2(nv, r1, a11), w22 = fma2(nx, r2, a22);
+    const F2 ntr = (w00 + w11 + w22) * F2(-2.0f / 3.0f);
+    // -tau
+    const F2 t00 = nmi * fma2(w00, F2(2.0f), ntr), t11 = nmi * fma2(w11, F2(2.0f), ntr),
+             t22 = nmi * fma2(w22, F2(2.0f), ntr);
+    const F2 t01 = nmi * (fma2(nu, r1, a01) + fma2(nv, r0, a10));
+    const F2 t02 = nmi * (fma2(nu, r2, a02) + fma2(nx, r0, a20));
+    const F2 t12 = nmi * (fma2(nv, r2, a12) + fma2(nx, r1, a21));
+    f.m00 = fma2(q1, u, t00) + p;
+    f.m11 = fma2(q2, v, t11) + p;
+    f.m22 = fma2(q3, x, t22) + p;
+    f.m01 = fma2(q1, v, t01);
+    f.m02 = fma2(q1, x, t02);
+    f.m12 = fma2(q2, x, t12);
+    const F2 nk = nmi * F2(gamma_over_pr<float>());
+    const F2 b0 = fma2(nx, a20, fma2(nv, a10, fma2(nu, a00, fma2(ce, r0, g(12)))));
+    f.e[0] = fma2(nk, b0, fma2(x, t02, fma2(v, t01, fma2(u, t00, h * u))));
+    const F2 b1 = fma2(nx, a21, fma2(nv, a11, fma2(nu, a01, fma2(ce, r1, g(13)))));
+    f.e[1] = fma2(nk, b1, fma2(x, t12, fma2(v, t11, fma2(u, t01, h * v))));
+    const F2 b2 = fma2(nx, a22, fma2(nv, a12, fma2(nu, a02, fma2(ce, r2, g(14)))));
+    f.e[2] = fma2(nk, b2, fma2(x, t22, fma2(v, t12, fma2(u, t02, h * x))));
+    return f;
+}
+
 // ---- the viscous terms of the kWideState pipelines, in the reference's order
 // (device_functions.cuh)
 

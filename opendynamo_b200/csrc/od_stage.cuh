@@ -1059,7 +1059,38 @@ __device__ __forceinline__ void stage_a_tile(const PA& A, unsigned char* smem_ra
     for (int v = 0; v < NV; ++v)
 #pragma unroll
         for (int a = 0; a < 4; ++a) divx[v][a] = !M::kWideState && v == 1 ? A.forcing : (C)0;
-    {
+    if constexpr (kLineUpdate<M, P, C>) {
+        // two points of the line at a time, in packed arithmetic (64-bit shared
+        // accesses; the pair is rotated by k's high bit so that the 16 lanes
+        // of an element hit distinct banks)
+        const int hk = l >> 3;
+#pragma unroll 1
+        for (int it = 0; it < 2; ++it) {
+            const int i = 2 * (it ^ hk);
+            const int p = li.c.x + i;
+            const VolumeFluxes2 F = volume_fluxes2<M>(
+                [&](int v) { return F2(*reinterpret_cast<const float2*>(&sm.u[v][p])); },
+                [&](int c) { return F2(*reinterpret_cast<const float2*>(&sm.g[c][p])); }, A.mu, A.suth);
+            auto put = [&](int row, const F2& x) { *reinterpret_cast<float2*>(&sm.g[row][p]) = x.v; };
+            const float2 q1 = *reinterpret_cast<const float2*>(&sm.u[1][p]);
+            put(kFy1, F.m01);
+            put(kFy2, F.m11);
+            put(kFy3, F.m12);
+            put(kFy4, F.e[1]);
+            put(kFz1, F.m02);
+            put(kFz3, F.m22);
+            put(kFz4, F.e[2]);
+#pragma unroll
+            for (int a = 0; a < 4; ++a) {
+                const float d0 = A.sc.nd[0][a * 4 + i], d1 = A.sc.nd[0][a * 4 + i + 1];
+                divx[0][a] = fma(d1, q1.y, fma(d0, q1.x, divx[0][a]));
+                divx[1][a] = fma(d1, F.m00.v.y, fma(d0, F.m00.v.x, divx[1][a]));
+                divx[2][a] = fma(d1, F.m01.v.y, fma(d0, F.m01.v.x, divx[2][a]));
+                divx[3][a] = fma(d1, F.m02.v.y, fma(d0, F.m02.v.x, divx[3][a]));
+                divx[4][a] = fma(d1, F.e[0].v.y, fma(d0, F.e[0].v.x, divx[4][a]));
+            }
+        }
+    } else {
         const int lk = l >> 2;
 #pragma unroll 1
         for (int it = 0; it < 4; ++it) {
