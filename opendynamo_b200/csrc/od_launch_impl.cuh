@@ -2,6 +2,7 @@
 // od_inst_*.cu translation units only.
 #pragma once
 
+#include <cstdint>
 #include <type_traits>
 
 #include "od_launch.h"
@@ -59,10 +60,24 @@ using MathFor = std::conditional_t<sizeof(S) == 8 && sizeof(C) == 4, WideState<M
 template <class S, class P, class C, class M>
 cudaError_t launch_a_flux(const StageAParams<S, P, C>& A, int flux, long long nelem, int epb, cudaStream_t s,
                           bool feat) {
+    // a caller's state (od_rhs_noalloc) may be less than 32-byte aligned: the
+    // kernels of 2 elements use 16-byte loads (40^3 f64 step 1.59 ms with 128-bit
+    // loads, 1.55 with 256-bit ones; u64/c32 1.9% faster, mixed 1.5%)
+    const bool narrow = sizeof(S) == 8 && (reinterpret_cast<uintptr_t>(A.u_in) & 31) != 0;
+    if (narrow) epb = 2;
     if (A.suth >= (C)0) {
-        // Sutherland variant: 4 elements per block only, no feature writing
+        // Sutherland variant: 4 elements per block (2 only for that case), no feature writing
         if (feat) return cudaErrorInvalidValue;
         using MS = WithSutherland<M>;
+        if constexpr (sizeof(S) == 8) {
+            if (narrow) {
+                switch (flux) {
+                    case kSlau2: return launch_a<S, P, C, MS, kSlau2, 2>(A, nelem, s);
+                    case kAusmPlus: return launch_a<S, P, C, MS, kAusmPlus, 2>(A, nelem, s);
+                    default: return launch_a<S, P, C, MS, kRusanov, 2>(A, nelem, s);
+                }
+            }
+        }
         switch (flux) {
             case kSlau2: return launch_a<S, P, C, MS, kSlau2, 4>(A, nelem, s);
             case kAusmPlus: return launch_a<S, P, C, MS, kAusmPlus, 4>(A, nelem, s);
@@ -180,6 +195,11 @@ cudaError_t prepare_flux() {
                                          cudaFuncAttributeMaxDynamicSharedMemorySize,
                                          (int)(sizeof(SlotFor<M, P, C>) * 2));
     if (e != cudaSuccess) return e;
+    if constexpr (sizeof(S) == 8) {
+        e = cudaFuncSetAttribute(stage_a_kernel<S, P, C, WithSutherland<M>, FLUX, 2>,
+                                 cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(sizeof(SlotFor<M, P, C>) * 2));
+        if (e != cudaSuccess) return e;
+    }
     e = cudaFuncSetAttribute(stage_a_kernel<S, P, C, WithSutherland<M>, FLUX, 4>,
                              cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(sizeof(SlotFor<M, P, C>) * 4));
     if (e != cudaSuccess) return e;

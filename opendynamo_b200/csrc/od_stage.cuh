@@ -250,6 +250,19 @@ __device__ __forceinline__ void ldg4(const S* __restrict__ p, P* q) {
     }
 }
 
+// the same of a 32-byte aligned f64 line in one 256-bit load (W): two 128-bit
+// loads of a warp's 16-byte halves touch every sector twice
+template <bool W, class S, class P>
+__device__ __forceinline__ void ldg4w(const S* __restrict__ p, P* q) {
+    if constexpr (W && sizeof(S) == 8) {
+        double a, b, c, d;
+        asm("ld.global.nc.v4.f64 {%0,%1,%2,%3}, [%4];" : "=d"(a), "=d"(b), "=d"(c), "=d"(d) : "l"(p));
+        q[0] = (P)a; q[1] = (P)b; q[2] = (P)c; q[3] = (P)d;
+    } else {
+        ldg4<S, P>(p, q);
+    }
+}
+
 // coherent 4-wide load (for data the same kernel later overwrites)
 template <class S, class P>
 __device__ __forceinline__ void ldc4(const S* p, P* q) {
@@ -607,7 +620,7 @@ __device__ __forceinline__ void viscous_face(const PA& A, Slot& sm, long long e,
 // the x and y gradients are in shared memory) also does the z faces' viscous
 // part (P5 for z): its normal gradient components are traced from registers
 // and the z-face corrections are stored once, complete.
-template <class M, int FLUX, int D, class PA, class Slot, class P = typename PA::P_t, class C = typename PA::C_t>
+template <class M, int FLUX, int D, bool W, class PA, class Slot, class P = typename PA::P_t, class C = typename PA::C_t>
 __device__ __forceinline__ void line_pass(const PA& A, Slot& sm, long long e, int l, const LineSet<P, C>& li,
                                           bool live, const long long nb0, const long long nb1, P* oL, P* oR,
                                           C (&jd)[2][NV], C* fi, const P (&qx)[NV][4]) {
@@ -638,8 +651,8 @@ __device__ __forceinline__ void line_pass(const PA& A, Slot& sm, long long e, in
             trace4_lr(q[v], A.tp.eL, A.tp.eR, oL[v], oR[v]);
             const P refl = (v > 0 && v < 4) ? (P)-1.0 : (P)1.0;
             P wm[4] = {(P)0, (P)0, (P)0, (P)0}, wp[4] = {(P)0, (P)0, (P)0, (P)0};
-            if (nb0 >= 0) ldg4<S, P>(A.u_in + v * m.npts + nb0 * NE + 4 * l, wm);
-            if (nb1 >= 0) ldg4<S, P>(A.u_in + v * m.npts + nb1 * NE + 4 * l, wp);
+            if (nb0 >= 0) ldg4w<W, S, P>(A.u_in + v * m.npts + nb0 * NE + 4 * l, wm);
+            if (nb1 >= 0) ldg4w<W, S, P>(A.u_in + v * m.npts + nb1 * NE + 4 * l, wp);
 #pragma unroll
             for (int a = 0; a < 4; ++a) {
                 wm[a] *= cm;
@@ -659,7 +672,7 @@ __device__ __forceinline__ void line_pass(const PA& A, Slot& sm, long long e, in
             P w[4];
             const S* base = A.u_in + v * m.npts + nb0 * NE;
             if constexpr (D == 0) {
-                ldg4<S, P>(base + 4 * l, w);
+                ldg4w<W, S, P>(base + 4 * l, w);
             } else {
 #pragma unroll
                 for (int mm = 0; mm < 4; ++mm) w[mm] = (P)__ldg(base + line_pt<D>(l, mm));
@@ -672,7 +685,7 @@ __device__ __forceinline__ void line_pass(const PA& A, Slot& sm, long long e, in
             P w[4];
             const S* base = A.u_in + v * m.npts + nb1 * NE;
             if constexpr (D == 0) {
-                ldg4<S, P>(base + 4 * l, w);
+                ldg4w<W, S, P>(base + 4 * l, w);
             } else {
 #pragma unroll
                 for (int mm = 0; mm < 4; ++mm) w[mm] = (P)__ldg(base + line_pt<D>(l, mm));
@@ -993,6 +1006,11 @@ __device__ __forceinline__ void stage_a_update_lines(const PA& A, Slot& sm, long
     }
 }
 
+// Phase A of an f64 state reads its x-lines with 256-bit loads in the kernels
+// of 4 elements per block; the kernels of 2 take any 16-byte aligned state.
+template <class S, int EPB>
+constexpr bool kWideLoads = sizeof(S) == 8 && EPB == 4;
+
 // One tile of phase A: EPB elements starting at A.e0 + tile * EPB, LPE
 // threads each. Called by whole warps: an element's 16 threads are half of one,
 // so nothing here waits for the block's other warps.
@@ -1001,6 +1019,7 @@ __device__ __forceinline__ void stage_a_tile(const PA& A, unsigned char* smem_ra
     using S = typename PA::S_t;
     using P = typename PA::P_t;
     using C = typename PA::C_t;
+    constexpr bool W = kWideLoads<S, EPB>;
     const int l = threadIdx.x & (LPE - 1);
     const int es = threadIdx.x / LPE;
     const int swz = (es & 1) << 3;
@@ -1021,7 +1040,7 @@ __device__ __forceinline__ void stage_a_tile(const PA& A, unsigned char* smem_ra
 #pragma unroll
     for (int v = 0; v < NV; ++v) {
         if (live) {
-            ldg4<S, P>(A.u_in + v * m.npts + ec * NE + 4 * l, qx[v]);
+            ldg4w<W, S, P>(A.u_in + v * m.npts + ec * NE + 4 * l, qx[v]);
         } else {
 #pragma unroll
             for (int a = 0; a < 4; ++a) qx[v][a] = (P)1.0;
@@ -1036,10 +1055,10 @@ __device__ __forceinline__ void stage_a_tile(const PA& A, unsigned char* smem_ra
     C jx[2][NV];      // this x-line's x-face corrections
     C jy[2][NV], jz[2][NV];   // kLineUpdate: the y- and z-line's
     C fi[3][NV];      // interface fluxes at the minus faces of this thread's lines
-    line_pass<M, FLUX, 0>(A, sm, ec, l, li, live, nxm, nxp, tr[0][0], tr[0][1], jx, fi[0], qx);
-    line_pass<M, FLUX, 1>(A, sm, ec, l, li, live, nym, nyp, tr[1][0], tr[1][1], jy, fi[1], qx);
+    line_pass<M, FLUX, 0, W>(A, sm, ec, l, li, live, nxm, nxp, tr[0][0], tr[0][1], jx, fi[0], qx);
+    line_pass<M, FLUX, 1, W>(A, sm, ec, l, li, live, nym, nyp, tr[1][0], tr[1][1], jy, fi[1], qx);
     __syncwarp();   // the x and y gradients, read by the z faces
-    line_pass<M, FLUX, 2>(A, sm, ec, l, li, live, nzm, nzp, tr[2][0], tr[2][1], jz, fi[2], qx);
+    line_pass<M, FLUX, 2, W>(A, sm, ec, l, li, live, nzm, nzp, tr[2][0], tr[2][1], jz, fi[2], qx);
     __syncwarp();
 
     // ---- P5: viscous face fluxes of the x and y faces, face records (the z
