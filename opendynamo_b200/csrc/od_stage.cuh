@@ -1187,10 +1187,13 @@ constexpr int stage_a_min_blocks() {
 template <class S, class P, class C, class M, int FLUX, int EPB, bool FEAT = false>
 __global__ void __launch_bounds__(LPE * EPB, (stage_a_min_blocks<S, P, C, EPB>())) stage_a_kernel(const StageAParams<S, P, C> A) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
-    // the closure network launched next may start its prologue (and prefetch
-    // its weights) on SMs this grid no longer needs; it reads the features
-    // and the RHS only after griddepcontrol.wait, i.e. after this grid
-    if constexpr (FEAT) asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    // the kernel launched next may become resident on SMs this grid no longer
+    // needs; it reads nothing before griddepcontrol.wait, i.e. before this grid
+    // is complete (the closure network: its prologue and weight prefetch
+    // overlap). The wait here is for the kernel before, when this launch is
+    // its programmatic dependent.
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    asm volatile("griddepcontrol.wait;" ::: "memory");
     stage_a_tile<M, FLUX, EPB, FEAT>(A, smem_raw, blockIdx.x);
 }
 
@@ -1423,6 +1426,8 @@ __global__ void __launch_bounds__(LPE * EPB) stage_b_kernel(const StageBParams<S
 // (48^3 f32: phase B 120.9 -> 117.5 us, phase A 263.0 -> 262.4 us).
 template <class S, class P, class C, int EPB>
 __global__ void __launch_bounds__(LPE * NV * EPB) stage_b_split_kernel(const StageBParams<S, P, C> B) {
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");   // as phase A
+    asm volatile("griddepcontrol.wait;" ::: "memory");
     const int g = threadIdx.x / LPE;
     const int v = g / EPB;
     const long long e = B.e0 + (long long)(gridDim.x - 1 - blockIdx.x) * EPB + (g - v * EPB);
