@@ -435,6 +435,7 @@ __device__ __forceinline__ uint4 pool8(const bf16* p) {
 template <bool VEC>
 __global__ void __launch_bounds__(256) gather_kernel(const bf16* __restrict__ Xp, const long long* __restrict__ rows,
                                                      int mv, int M, bf16* __restrict__ X, bf16* __restrict__ XT) {
+    od::dependent_start();
     __shared__ __align__(16) bf16 tile[64 * 64];
     const int m0 = blockIdx.x * 64, c0 = blockIdx.y * 64;
 #pragma unroll
@@ -462,6 +463,7 @@ __global__ void __launch_bounds__(256) loss_grad_kernel(const float* __restrict_
                                                         const bf16* __restrict__ Tp, const long long* __restrict__ rows,
                                                         int M, int mv, float g, bf16* __restrict__ dY,
                                                         bf16* __restrict__ dYT, double* loss) {
+    od::dependent_start();
     __shared__ __align__(16) bf16 tile[64 * 64];
     __shared__ double red[8];
     const int m0 = blockIdx.x * 64, n0 = blockIdx.y * 64;
@@ -570,6 +572,7 @@ __device__ __forceinline__ float row_sum(const bf16* AT, int M, int n, int lane)
 }
 
 __global__ void __launch_bounds__(kFinishThreads) grad_finish_kernel(const GradFinish F) {
+    od::dependent_start();
     const int b = (int)blockIdx.x;
     if (b < F.first_b[4]) {
         int l = 0;
@@ -624,6 +627,7 @@ constexpr int kAdamRows = 32;   // rows of a weight tile (of 64 columns)
 // layers' biases. (Eight launches of one value a thread with 2-byte stores
 // into W^T, and a ninth for the image, took 39 us; this one 9 us.)
 __global__ void __launch_bounds__(256) adam_kernel(const AdamArgs A, int tiles) {
+    od::dependent_start();
     __shared__ __align__(16) bf16 tile[kAdamRows * 64];
     int b = blockIdx.x, l = 0;
     if (b >= tiles) {
@@ -781,9 +785,8 @@ cudaError_t backward(od_mlp* m, const bf16* XT, int M, int mv, const bf16* Tp) {
     const float gs = 2.0f / ((float)mv * (float)kOut);
     auto* lg = !Tp ? loss_grad_kernel<false, true>
                    : aligned16(Tp) ? loss_grad_kernel<true, true> : loss_grad_kernel<true, false>;
-    lg<<<dim3(M / 64, kOutPad / 64), 256, 0, m->stream>>>(m->Y, m->T, Tp, m->rows_d, M, mv, gs, m->dY, m->dYT,
-                                                          m->loss);
-    if (e == cudaSuccess) e = cudaGetLastError();
+    e = od::launch_dependent(true, lg, dim3(M / 64, kOutPad / 64), 256, 0, m->stream, m->Y, m->T, Tp, m->rows_d, M, mv,
+                             gs, m->dY, m->dYT, m->loss);
     // down the layers: dZ of the hidden layers, each with its transposed copy
     const bf16* dz = m->dY;
     for (int l = 2; l >= 0 && e == cudaSuccess; --l) {
@@ -821,8 +824,7 @@ cudaError_t backward(od_mlp* m, const bf16* XT, int M, int mv, const bf16* Tp) {
         if (g[l].ksplit > 1) nb += (int)(F.mn[l] / kFinishThreads);
     }
     F.first_w[4] = nb;
-    grad_finish_kernel<<<(unsigned)nb, kFinishThreads, 0, m->stream>>>(F);
-    return cudaGetLastError();
+    return od::launch_dependent(true, grad_finish_kernel, (unsigned)nb, kFinishThreads, 0, m->stream, F);
 }
 
 constexpr size_t kStatusBytes = 16;   // loss and err, cleared and read back together
@@ -1032,8 +1034,7 @@ int od_mlp_train_step(od_mlp* m, const void* Xpool, const void* Tpool, const lon
         tiles += (m->rows[l] / kAdamRows) * (m->cols[l] / 64);
     }
     if (e == cudaSuccess) {
-        adam_kernel<<<tiles + 4, 256, 0, m->stream>>>(A, tiles);
-        e = cudaGetLastError();
+        e = od::launch_dependent(true, adam_kernel, tiles + 4, 256, 0, m->stream, A, tiles);
     }
     if (e != cudaSuccess) return mfail(m, OD_ERR_CUDA, cudaGetErrorString(e));
     double l = 0;

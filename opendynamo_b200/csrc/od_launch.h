@@ -7,6 +7,34 @@
 
 namespace od {
 
+// Launches fn; dependent: as a programmatic dependent of the kernel before it
+// on the stream. The kernel then may be resident before that one has finished
+// and has to execute griddepcontrol.wait before it touches memory.
+template <class... P, class... A>
+cudaError_t launch_dependent(bool dependent, void (*fn)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t s,
+                             A&&... args) {
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = grid;
+    cfg.blockDim = block;
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = s;
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = at;
+    cfg.numAttrs = dependent ? 1 : 0;
+    return cudaLaunchKernelEx(&cfg, fn, static_cast<P>(args)...);
+}
+
+#ifdef __CUDACC__
+// Waits for the kernel this one is a programmatic dependent of (none: returns
+// at once) and lets the kernel after this one become resident.
+__device__ __forceinline__ void dependent_start() {
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+}
+#endif
+
 enum StageFlags : int {
     kHasU0 = 1,      // out = ra*u0 + rb*u_in + rc*R (else rb*u_in + rc*R)
     kRoundQ = 2,     // round the gradient through f32 (q_real = f32 with f64 compute)

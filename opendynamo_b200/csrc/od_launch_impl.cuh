@@ -39,22 +39,6 @@ constexpr bool has_feat_variant() {
 // at 8 to 16, 1.2% at 32, nothing at 48; but u64/c32 2% slower at 48 and 64.
 constexpr long long kDependentElems = 1 << 16;
 
-template <class Params>
-cudaError_t launch_stage_kernel(void (*fn)(Params), unsigned grid, unsigned block, size_t smem, cudaStream_t s,
-                                long long nelem, const Params& p) {
-    cudaLaunchConfig_t cfg{};
-    cfg.gridDim = dim3(grid);
-    cfg.blockDim = dim3(block);
-    cfg.dynamicSmemBytes = smem;
-    cfg.stream = s;
-    cudaLaunchAttribute at[1];
-    at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    at[0].val.programmaticStreamSerializationAllowed = 1;
-    cfg.attrs = at;
-    cfg.numAttrs = nelem <= kDependentElems ? 1 : 0;
-    return cudaLaunchKernelEx(&cfg, fn, p);
-}
-
 template <class S, class P, class C, class M, int FLUX, int EPB>
 cudaError_t launch_a(const StageAParams<S, P, C>& A, long long nelem, cudaStream_t s, bool feat = false) {
     const unsigned grid = (unsigned)((nelem + EPB - 1) / EPB);
@@ -62,11 +46,12 @@ cudaError_t launch_a(const StageAParams<S, P, C>& A, long long nelem, cudaStream
     const size_t smem = sizeof(SlotFor<M, P, C>) * EPB;
     if constexpr (has_feat_variant<S, P, C, M>() && EPB == 4) {
         if (feat) {
-            return launch_stage_kernel(stage_a_kernel<S, P, C, M, FLUX, EPB, true>, grid, LPE * EPB, smem, s, nelem, A);
+            return launch_dependent(nelem <= kDependentElems, stage_a_kernel<S, P, C, M, FLUX, EPB, true>, grid,
+                                    LPE * EPB, smem, s, A);
         }
     }
     if (feat) return cudaErrorInvalidValue;   // no variant writes the features for this launch
-    return launch_stage_kernel(stage_a_kernel<S, P, C, M, FLUX, EPB>, grid, LPE * EPB, smem, s, nelem, A);
+    return launch_dependent(nelem <= kDependentElems, stage_a_kernel<S, P, C, M, FLUX, EPB>, grid, LPE * EPB, smem, s, A);
 }
 
 template <class S, class P, class C, class M, int FLUX>
@@ -125,7 +110,7 @@ template <class S, class P, class C, int EPB>
 cudaError_t launch_b_split(const StageBParams<S, P, C>& B, long long nelem, cudaStream_t s) {
     const unsigned grid = (unsigned)((nelem + EPB - 1) / EPB);
     if (grid == 0) return cudaSuccess;
-    return launch_stage_kernel(stage_b_split_kernel<S, P, C, EPB>, grid, LPE * NV * EPB, 0, s, nelem, B);
+    return launch_dependent(nelem <= kDependentElems, stage_b_split_kernel<S, P, C, EPB>, grid, LPE * NV * EPB, 0, s, B);
 }
 
 // fast math changes only f32 arithmetic: f64-compute combinations use one variant

@@ -44,8 +44,7 @@ cudaError_t launch_gemm_t(const GemmArgs& g, cudaStream_t s) {
     }
     const int ks = g.ksplit > 1 ? g.ksplit : 1;
     dim3 grid((unsigned)(g.M / BM), (unsigned)(g.N / NT), (unsigned)ks);
-    gemm_kernel<NT, EPI><<<grid, kGemmThreads, smem, s>>>(g);
-    e = cudaGetLastError();
+    e = launch_dependent(true, gemm_kernel<NT, EPI>, grid, kGemmThreads, smem, s, g);
     if (e == cudaSuccess && ks > 1) {
         const long long mn = (long long)g.M * g.N;
         splitk_reduce_kernel<<<(unsigned)((mn + 127) / 128), 128, 0, s>>>(g.ws, ks, mn, g.N, g.bias, g.out_f32);
@@ -114,8 +113,7 @@ cudaError_t launch_gemm_group(GemmArgs* g, int n, float* ws, size_t ws_floats, c
         if (e != cudaSuccess) return e;
         prepared[dev] = true;
     }
-    gemm_group_kernel<<<(unsigned)ctas, kGemmThreads, smem, s>>>(q);
-    return cudaGetLastError();
+    return launch_dependent(true, gemm_group_kernel, (unsigned)ctas, kGemmThreads, smem, s, q);
 }
 
 // C = A B^T with the epilogue `epi`; M % 128 == 0, N % 64 == 0, K % 64 == 0.

@@ -28,6 +28,8 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include "od_launch.h"
+
 namespace od {
 namespace mlp {
 
@@ -313,6 +315,9 @@ __device__ __forceinline__ void gemm_tile(const GemmArgs& g, int bx, int by, int
     const uint32_t tmem = s.tmem_base;
     const uint32_t idesc = instr_desc(BM, NT);
 
+    // launched as a programmatic dependent: the set-up above overlaps the end
+    // of the kernel before, whose results are read from here on
+    dependent_start();
     // prologue: blocks 0 .. STAGES-1, one cp.async group each (empty groups
     // past the end keep the group count)
     const LoadPos pos = load_pos(g, m0, n0, kb0);

@@ -1192,8 +1192,7 @@ __global__ void __launch_bounds__(LPE * EPB, (stage_a_min_blocks<S, P, C, EPB>()
     // is complete (the closure network: its prologue and weight prefetch
     // overlap). The wait here is for the kernel before, when this launch is
     // its programmatic dependent.
-    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
-    asm volatile("griddepcontrol.wait;" ::: "memory");
+    dependent_start();
     stage_a_tile<M, FLUX, EPB, FEAT>(A, smem_raw, blockIdx.x);
 }
 
@@ -1426,8 +1425,7 @@ __global__ void __launch_bounds__(LPE * EPB) stage_b_kernel(const StageBParams<S
 // (48^3 f32: phase B 120.9 -> 117.5 us, phase A 263.0 -> 262.4 us).
 template <class S, class P, class C, int EPB>
 __global__ void __launch_bounds__(LPE * NV * EPB) stage_b_split_kernel(const StageBParams<S, P, C> B) {
-    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");   // as phase A
-    asm volatile("griddepcontrol.wait;" ::: "memory");
+    dependent_start();   // as phase A
     const int g = threadIdx.x / LPE;
     const int v = g / EPB;
     const long long e = B.e0 + (long long)(gridDim.x - 1 - blockIdx.x) * EPB + (g - v * EPB);
