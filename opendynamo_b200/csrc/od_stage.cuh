@@ -335,14 +335,15 @@ __device__ __forceinline__ void st_xline(T* row, int x, const T* q) {
     }
 }
 
-// Whether every face correction of a line stays in its thread's registers
-// (the all-f32 kernels): the update then works on the thread's own y- and
-// z-lines, one row line in and one out per variable, where the update of a
-// whole x-line loads the four x-lines of its k-plane and of its j-column and
-// the corrections of four lines (960 bytes a thread, a third of the kernel's
-// shared-memory traffic). f64 needs the registers.
+// Whether every face correction of a line stays in its thread's registers (all
+// but the kWideState pipelines, whose operation order the other update keeps):
+// the update then works on the thread's own y- and z-lines, one row line in
+// and one out per variable, where the update of a whole x-line loads the four
+// x-lines of its k-plane and of its j-column and the corrections of four lines
+// (a third of the kernel's shared-memory traffic). 48^3 f32 step 1.10 -> 1.06
+// ms, 40^3 f64 1.55 -> 1.46.
 template <class M, class P, class C>
-constexpr bool kLineUpdate = !M::kWideState && sizeof(P) == 4 && sizeof(C) == 4;
+constexpr bool kLineUpdate = !M::kWideState && sizeof(P) == sizeof(C);
 
 template <class P, class C, bool J>
 struct SlotBytes {
@@ -958,50 +959,78 @@ __device__ __forceinline__ void stage_a_update(const PA& A, Slot& sm, long long 
 // direction. Called by whole warps.
 constexpr int kR = 7;   // first row of the partial updates (rows 0-6: the fluxes)
 
+// r += the divergence (DIV) and / or the lifting (LIFT) of the thread's
+// direction-D line of variable v; f: the line's fluxes, j0, j1: its faces' corrections
+template <int D, bool DIV, bool LIFT, class PA, class C>
+__device__ __forceinline__ void line_terms(const PA& A, const C* f, C j0, C j1, C* r) {
+#pragma unroll
+    for (int a = 0; a < 4; ++a) {
+        if constexpr (LIFT) {
+            r[a] = fma(j0, A.sc.nl[D][a], r[a]);
+            r[a] = fma(j1, A.sc.nr[D][a], r[a]);
+        }
+        if constexpr (DIV) {
+#pragma unroll
+            for (int mm = 0; mm < 4; ++mm) r[a] = fma(A.sc.nd[D][a * 4 + mm], f[mm], r[a]);
+        }
+    }
+}
+
+// One pass of the update over the thread's direction-D lines (y or z): rows kR..
+// FRESH: they start here.
+template <class M, int D, bool FRESH, bool DIV, bool LIFT, class PA, class Slot, class L, class C>
+__device__ __forceinline__ void update_pass(const PA& A, Slot& sm, const L& li, const C (&j)[2][NV]) {
+#pragma unroll
+    for (int v = 0; v < NV; ++v) {
+        C f[4], r[4] = {(C)0, (C)0, (C)0, (C)0};
+        if constexpr (DIV) row_line_load<D>(flux_row<M, D>(sm, v), li, f);
+        if constexpr (!FRESH) row_line_load<D>(&sm.g[kR + v][0], li, r);
+        line_terms<D, DIV, LIFT>(A, f, j[0][v], j[1][v], r);
+        row_line_store<D>(&sm.g[kR + v][0], li, r);
+    }
+    __syncwarp();
+}
+
 template <class M, class PA, class Slot, class P = typename PA::P_t, class C = typename PA::C_t>
 __device__ __forceinline__ void stage_a_update_lines(const PA& A, Slot& sm, long long ec, int l,
                                                      const LineSet<P, C>& li, bool live, const C (&divx)[NV][4],
                                                      const C (&jx)[2][NV], const C (&jy)[2][NV],
                                                      const C (&jz)[2][NV]) {
+    if constexpr (sizeof(C) == 8) {
+        if (A.flags & kRoundRhs) {
+            // the volume terms of all directions are rounded before the lifting
+            update_pass<M, 1, true, true, false>(A, sm, li, jy);
+            update_pass<M, 2, false, true, false>(A, sm, li, jz);
 #pragma unroll
-    for (int v = 0; v < NV; ++v) {
-        C f[4], r[4];
-        row_line_load<1>(flux_row<M, 1>(sm, v), li, f);
+            for (int v = 0; v < NV; ++v) {
+                C r[4];
+                row_line_load<0>(&sm.g[kR + v][0], li, r);
 #pragma unroll
-        for (int a = 0; a < 4; ++a) {
-            r[a] = jy[0][v] * A.sc.nl[1][a];
-            r[a] = fma(jy[1][v], A.sc.nr[1][a], r[a]);
+                for (int a = 0; a < 4; ++a) r[a] = (C)(float)(r[a] + divx[v][a]);
+                line_terms<0, false, true>(A, r, jx[0][v], jx[1][v], r);
+                row_line_store<0>(&sm.g[kR + v][0], li, r);
+            }
+            __syncwarp();
+            update_pass<M, 1, false, false, true>(A, sm, li, jy);
+            update_pass<M, 2, false, false, true>(A, sm, li, jz);
 #pragma unroll
-            for (int mm = 0; mm < 4; ++mm) r[a] = fma(A.sc.nd[1][a * 4 + mm], f[mm], r[a]);
+            for (int v = 0; v < NV; ++v) {
+                C r[4];
+                row_line_load<0>(&sm.g[kR + v][0], li, r);
+                if (live) store_update(A, ec, l, v, r);
+            }
+            return;
         }
-        row_line_store<1>(sm.g[kR + v], li, r);
     }
-    __syncwarp();
-#pragma unroll
-    for (int v = 0; v < NV; ++v) {
-        C f[4], r[4];
-        row_line_load<2>(flux_row<M, 2>(sm, v), li, f);
-        row_line_load<2>(sm.g[kR + v], li, r);
-#pragma unroll
-        for (int a = 0; a < 4; ++a) {
-            r[a] = fma(jz[0][v], A.sc.nl[2][a], r[a]);
-            r[a] = fma(jz[1][v], A.sc.nr[2][a], r[a]);
-#pragma unroll
-            for (int mm = 0; mm < 4; ++mm) r[a] = fma(A.sc.nd[2][a * 4 + mm], f[mm], r[a]);
-        }
-        row_line_store<2>(sm.g[kR + v], li, r);
-    }
-    __syncwarp();
+    update_pass<M, 1, true, true, true>(A, sm, li, jy);
+    update_pass<M, 2, false, true, true>(A, sm, li, jz);
 #pragma unroll
     for (int v = 0; v < NV; ++v) {
         C r[4];
-        row_line_load<0>(sm.g[kR + v], li, r);
+        row_line_load<0>(&sm.g[kR + v][0], li, r);
 #pragma unroll
-        for (int a = 0; a < 4; ++a) {
-            r[a] += divx[v][a];
-            r[a] = fma(jx[0][v], A.sc.nl[0][a], r[a]);
-            r[a] = fma(jx[1][v], A.sc.nr[0][a], r[a]);
-        }
+        for (int a = 0; a < 4; ++a) r[a] += divx[v][a];
+        line_terms<0, false, true>(A, r, jx[0][v], jx[1][v], r);
         if (live) store_update(A, ec, l, v, r);
     }
 }
@@ -1078,7 +1107,7 @@ __device__ __forceinline__ void stage_a_tile(const PA& A, unsigned char* smem_ra
     for (int v = 0; v < NV; ++v)
 #pragma unroll
         for (int a = 0; a < 4; ++a) divx[v][a] = !M::kWideState && v == 1 ? A.forcing : (C)0;
-    if constexpr (kLineUpdate<M, P, C>) {
+    if constexpr (kLineUpdate<M, P, C> && sizeof(C) == 4) {
         // two points of the line at a time, in packed arithmetic (64-bit shared
         // accesses; the pair is rotated by k's high bit so that the 16 lanes
         // of an element hit distinct banks)
