@@ -179,6 +179,7 @@ cudaError_t launch_stage_t(const StageLaunch& L, cudaStream_t s) {
         B.rb = A.rb;
         B.rc = A.rc;
         B.flags = A.flags;
+        if (sizeof(S) == 8 && (reinterpret_cast<uintptr_t>(L.u_out) & 31) == 0) B.flags |= kWideOut;
         B.e0 = L.e0;
         B.e1 = L.e1;
         if (L.epb_b == 8)

@@ -272,6 +272,21 @@ __device__ __forceinline__ void ldc4(const S* p, P* q) {
     for (int a = 0; a < 4; ++a) q[a] = (P)w[a];
 }
 
+// coherent 256-bit load / store of a 32-byte aligned f64 line
+template <class S, class P>
+__device__ __forceinline__ void ld4wide(const S* p, P* q) {
+    double a, b, c, d;
+    asm volatile("ld.global.v4.f64 {%0,%1,%2,%3}, [%4];" : "=d"(a), "=d"(b), "=d"(c), "=d"(d) : "l"(p) : "memory");
+    q[0] = (P)a; q[1] = (P)b; q[2] = (P)c; q[3] = (P)d;
+}
+
+template <class S, class P>
+__device__ __forceinline__ void st4wide(S* p, const P* q) {
+    asm volatile("st.global.v4.f64 [%4], {%0,%1,%2,%3};" ::"d"((double)q[0]), "d"((double)q[1]), "d"((double)q[2]),
+                 "d"((double)q[3]), "l"(p)
+                 : "memory");
+}
+
 template <class S, class P>
 __device__ __forceinline__ void stg4(S* p, const P* q) {
     if constexpr (sizeof(S) == 4) {
@@ -1264,11 +1279,19 @@ __device__ __forceinline__ T ldf(const T* p) {
 }
 
 // 4-wide load of data read once (evict-first: the face records and the RHS
-// phase B consumes), or coherent inside a persistent kernel (COH)
+// phase B consumes, in buffers of this library: 32-byte aligned lines), or
+// coherent inside a persistent kernel (COH)
 template <bool COH, class S, class P>
 __device__ __forceinline__ void ld4once(const S* p, P* q) {
-    if constexpr (COH || sizeof(S) != 4) {
+    if constexpr (COH) {
         ldc4<S, P>(p, q);
+    } else if constexpr (sizeof(S) == 8) {
+        double a, b, c, d;
+        asm volatile("ld.global.cs.v4.f64 {%0,%1,%2,%3}, [%4];"
+                     : "=d"(a), "=d"(b), "=d"(c), "=d"(d)
+                     : "l"(p)
+                     : "memory");
+        q[0] = (P)a; q[1] = (P)b; q[2] = (P)c; q[3] = (P)d;
     } else {
         const float4 v = __ldcs(reinterpret_cast<const float4*>(p));
         q[0] = (P)v.x; q[1] = (P)v.y; q[2] = (P)v.z; q[3] = (P)v.w;
@@ -1380,6 +1403,8 @@ __device__ __forceinline__ BVar<P, C> b_load(const PB& B, const BCtx<C>& x, int 
         ld4once<COH, S, C>(B.rhs + off, d.r);
         ldg4<S, P>(B.u_in + off, d.un);
         if (B.flags & kHasU0) ldc4<S, P>(B.u0 + off, d.u0);
+    } else if (sizeof(S) == 8 && (B.flags & kWideOut)) {
+        ld4wide(B.u_out + off, d.un);
     } else {
         ldc4<S, P>(B.u_out + off, d.un);
     }
@@ -1404,7 +1429,10 @@ __device__ __forceinline__ void b_store(const PB& B, const BCtx<C>& x, int v, co
 #pragma unroll
         for (int i = 0; i < 4; ++i) out[i] = d.un[i] + B.rc * (P)d.acc[i];
     }
-    stg4<S, P>(B.u_out + off, out);
+    if (sizeof(S) == 8 && (B.flags & kWideOut))
+        st4wide(B.u_out + off, out);
+    else
+        stg4<S, P>(B.u_out + off, out);
 }
 
 template <bool COH, class PB, class C = typename PB::C_t>
