@@ -228,6 +228,29 @@ struct FeatParams {
     float mean[kChan], inv_scale[kChan];
 };
 
+// The standardised features of a point from its conserved variables c and
+// their derivatives d[var][direction]: (value - mean) / scale, clipped, as
+// bf16. Every rounding is pinned (no contraction is left to the compiler):
+// phase A writes the same features (stage_a_features), value for value.
+template <class Put>
+__device__ __forceinline__ void feature_channels(const FeatParams& fp, const float* c, const float (&d)[4][3], Put put) {
+    auto emit = [&](int i, float x) {   // x: the channel minus its mean
+        put(i, __float2bfloat16_rn(fminf(fmaxf(__fmul_rn(x, fp.inv_scale[i]), -kClip), kClip)));
+    };
+    const float ir = 1.0f / c[0];
+#pragma unroll
+    for (int v = 0; v < 5; ++v) emit(v, __fadd_rn(c[v], -fp.mean[v]));
+#pragma unroll
+    for (int a = 0; a < 3; ++a) {
+        const float nu = __fmul_rn(c[1 + a], -ir);
+#pragma unroll
+        for (int b = 0; b < 3; ++b) {
+            const int i = 5 + 3 * a + b;
+            emit(i, __fmaf_rn(__fmaf_rn(nu, d[0][b], d[1 + a][b]), ir, -fp.mean[i]));
+        }
+    }
+}
+
 // X: row-major [element][channel * 64 + point]; a thread per point.
 template <class T>
 __global__ void __launch_bounds__(64) features_kernel(const T* __restrict__ u, FeatParams fp, bf16* __restrict__ X) {
@@ -247,27 +270,16 @@ __global__ void __launch_bounds__(64) features_kernel(const T* __restrict__ u, F
         float sx = 0.f, sy = 0.f, sz = 0.f;
 #pragma unroll
         for (int m = 0; m < 4; ++m) {
-            sx += fp.D[i * 4 + m] * q[v][m + 4 * j + 16 * k];
-            sy += fp.D[j * 4 + m] * q[v][i + 4 * m + 16 * k];
-            sz += fp.D[k * 4 + m] * q[v][i + 4 * j + 16 * m];
+            sx = __fmaf_rn(fp.D[i * 4 + m], q[v][m + 4 * j + 16 * k], sx);
+            sy = __fmaf_rn(fp.D[j * 4 + m], q[v][i + 4 * m + 16 * k], sy);
+            sz = __fmaf_rn(fp.D[k * 4 + m], q[v][i + 4 * j + 16 * m], sz);
         }
-        d[v][0] = sx * fp.jac[0];
-        d[v][1] = sy * fp.jac[1];
-        d[v][2] = sz * fp.jac[2];
+        d[v][0] = __fmul_rn(sx, fp.jac[0]);
+        d[v][1] = __fmul_rn(sy, fp.jac[1]);
+        d[v][2] = __fmul_rn(sz, fp.jac[2]);
     }
-    const float ir = 1.0f / c[0];
-    float ch[kChan];
-#pragma unroll
-    for (int v = 0; v < 5; ++v) ch[v] = c[v];
-#pragma unroll
-    for (int a = 0; a < 3; ++a)
-#pragma unroll
-        for (int b = 0; b < 3; ++b) ch[5 + 3 * a + b] = (d[1 + a][b] - c[1 + a] * ir * d[0][b]) * ir;
     bf16* row = X + e * kIn + p;
-#pragma unroll
-    for (int ch_i = 0; ch_i < kChan; ++ch_i)
-        row[ch_i * 64] = __float2bfloat16_rn(fminf(fmaxf((ch[ch_i] - fp.mean[ch_i]) * fp.inv_scale[ch_i], -kClip),
-                                                   kClip));
+    feature_channels(fp, c, d, [&](int ch, bf16 x) { row[ch * 64] = x; });
 }
 
 // The same features for the fused inference kernel, written in its layout:
@@ -303,7 +315,7 @@ __global__ void __launch_bounds__(16 * kFeatEpb) features_tiled_kernel(const flo
         if (v < 4) *reinterpret_cast<float4*>(&q[es][v][4 * l]) = w;
     }
     __syncthreads();
-    float d[4][3][4];   // [var][direction][point of the line]
+    float d[4][4][3];   // [point of the line][var][direction]
 #pragma unroll
     for (int v = 0; v < 4; ++v) {
         float ly[4][4], lz[4][4];   // the x-lines (m, k) and (j, m), m = 0..3
@@ -319,30 +331,20 @@ __global__ void __launch_bounds__(16 * kFeatEpb) features_tiled_kernel(const flo
             float sx = 0.f, sy = 0.f, sz = 0.f;
 #pragma unroll
             for (int m = 0; m < 4; ++m) {
-                sx += fp.D[i * 4 + m] * c[v][m];
-                sy += fp.D[j * 4 + m] * ly[m][i];
-                sz += fp.D[k * 4 + m] * lz[m][i];
+                sx = __fmaf_rn(fp.D[i * 4 + m], c[v][m], sx);
+                sy = __fmaf_rn(fp.D[j * 4 + m], ly[m][i], sy);
+                sz = __fmaf_rn(fp.D[k * 4 + m], lz[m][i], sz);
             }
-            d[v][0][i] = sx * fp.jac[0];
-            d[v][1][i] = sy * fp.jac[1];
-            d[v][2][i] = sz * fp.jac[2];
+            d[i][v][0] = __fmul_rn(sx, fp.jac[0]);
+            d[i][v][1] = __fmul_rn(sy, fp.jac[1]);
+            d[i][v][2] = __fmul_rn(sz, fp.jac[2]);
         }
     }
 #pragma unroll
     for (int i = 0; i < 4; ++i) {
         const int p = i + 4 * l;
-        const float ir = 1.0f / c[0][i];
-        float ch[kChan];
-#pragma unroll
-        for (int v = 0; v < 5; ++v) ch[v] = c[v][i];
-#pragma unroll
-        for (int a = 0; a < 3; ++a)
-#pragma unroll
-            for (int b = 0; b < 3; ++b) ch[5 + 3 * a + b] = (d[1 + a][b][i] - c[1 + a][i] * ir * d[0][b][i]) * ir;
-#pragma unroll
-        for (int ch_i = 0; ch_i < kChan; ++ch_i)
-            st[es][ch_i][p] = __float2bfloat16_rn(fminf(fmaxf((ch[ch_i] - fp.mean[ch_i]) * fp.inv_scale[ch_i], -kClip),
-                                                        kClip));
+        const float ci[5] = {c[0][i], c[1][i], c[2][i], c[3][i], c[4][i]};
+        feature_channels(fp, ci, d[i], [&](int ch, bf16 x) { st[es][ch][p] = x; });
     }
     __syncthreads();
     if (!live) return;
