@@ -130,6 +130,9 @@ cudaError_t launch_diag(const void* u, bool u_f64, int nx, int ny, int nz, doubl
 cudaError_t launch_stage_f32(const StageLaunch& L, cudaStream_t s);
 cudaError_t launch_stage_f64(const StageLaunch& L, cudaStream_t s);
 cudaError_t launch_stage_u64c32(const StageLaunch& L, cudaStream_t s);
+// the u64/c32 pipeline on a state held in f32 (od_ctx::narrow): the same kernels
+// and roundings with f32 storage
+cudaError_t launch_stage_u64c32_narrow(const StageLaunch& L, cudaStream_t s);
 cudaError_t launch_stage_u32c64(const StageLaunch& L, cudaStream_t s);
 cudaError_t launch_stage_mixed(const StageLaunch& L, cudaStream_t s);
 
@@ -137,6 +140,7 @@ cudaError_t launch_stage_mixed(const StageLaunch& L, cudaStream_t s);
 cudaError_t prepare_kernels_f32();
 cudaError_t prepare_kernels_f64();
 cudaError_t prepare_kernels_u64c32();
+cudaError_t prepare_kernels_u64c32_narrow();
 cudaError_t prepare_kernels_u32c64();
 cudaError_t prepare_kernels_mixed();
 

@@ -28,7 +28,7 @@ Tab<T> cast_tab(const TablesD& t) {
 // configuration); feat says whether this launch writes them.
 template <class S, class P, class C, class M>
 constexpr bool has_feat_variant() {
-    return sizeof(S) == 4 && sizeof(P) == 4 && sizeof(C) == 4 && !M::kSutherland;
+    return sizeof(S) == 4 && sizeof(P) == 4 && sizeof(C) == 4 && !M::kSutherland && !M::kWideState;
 }
 
 // Launches of small meshes are programmatic dependents of the kernel before
@@ -61,8 +61,9 @@ cudaError_t launch_a_epb(const StageAParams<S, P, C>& A, long long nelem, int ep
 }
 
 // f32 fluxes under an f64 state: the policy that keeps their operation order
-template <class S, class C, class M>
-using MathFor = std::conditional_t<sizeof(S) == 8 && sizeof(C) == 4, WideState<M>, M>;
+// (WIDE: such a state held in f32, launch_stage_u64c32_narrow)
+template <class S, class C, class M, bool WIDE>
+using MathFor = std::conditional_t<WIDE || (sizeof(S) == 8 && sizeof(C) == 4), WideState<M>, M>;
 
 template <class S, class P, class C, class M>
 cudaError_t launch_a_flux(const StageAParams<S, P, C>& A, int flux, long long nelem, int epb, cudaStream_t s,
@@ -117,7 +118,7 @@ cudaError_t launch_b_split(const StageBParams<S, P, C>& B, long long nelem, cuda
 template <class C>
 constexpr bool has_fast_variant() { return sizeof(C) == 4; }
 
-template <class S, class P, class C>
+template <class S, class P, class C, bool WIDE = false>
 cudaError_t launch_stage_t(const StageLaunch& L, cudaStream_t s) {
     StageAParams<S, P, C> A{};
     A.u_in = (const S*)L.u_in;
@@ -155,11 +156,11 @@ cudaError_t launch_stage_t(const StageLaunch& L, cudaStream_t s) {
         if (L.ev[0]) cudaEventRecord(L.ev[0], s);
         if constexpr (has_fast_variant<C>()) {
             if (L.fast_math)
-                err = launch_a_flux<S, P, C, MathFor<S, C, MathFast>>(A, L.flux, count, L.epb_a, s, feat);
+                err = launch_a_flux<S, P, C, MathFor<S, C, MathFast, WIDE>>(A, L.flux, count, L.epb_a, s, feat);
             else
-                err = launch_a_flux<S, P, C, MathFor<S, C, MathIeee>>(A, L.flux, count, L.epb_a, s, feat);
+                err = launch_a_flux<S, P, C, MathFor<S, C, MathIeee, WIDE>>(A, L.flux, count, L.epb_a, s, feat);
         } else {
-            err = launch_a_flux<S, P, C, MathFor<S, C, MathIeee>>(A, L.flux, count, L.epb_a, s, feat);
+            err = launch_a_flux<S, P, C, MathFor<S, C, MathIeee, WIDE>>(A, L.flux, count, L.epb_a, s, feat);
         }
         if (err != cudaSuccess) return err;
         if (L.ev[1]) cudaEventRecord(L.ev[1], s);
@@ -223,11 +224,11 @@ cudaError_t prepare_m() {
     return prepare_flux<S, P, C, M, kRusanov>();
 }
 
-template <class S, class P, class C>
+template <class S, class P, class C, bool WIDE = false>
 cudaError_t prepare_t() {
-    cudaError_t e = prepare_m<S, P, C, MathFor<S, C, MathIeee>>();
+    cudaError_t e = prepare_m<S, P, C, MathFor<S, C, MathIeee, WIDE>>();
     if constexpr (has_fast_variant<C>()) {
-        if (e == cudaSuccess) e = prepare_m<S, P, C, MathFor<S, C, MathFast>>();
+        if (e == cudaSuccess) e = prepare_m<S, P, C, MathFor<S, C, MathFast, WIDE>>();
     }
     return e;
 }
