@@ -197,8 +197,8 @@ __device__ __forceinline__ T sum4_scatter(const T (&p)[4], int q) {
     return d + __shfl_xor_sync(0xffffffffu, e, 1);
 }
 
-// neighbour across face (d, side) or -1 for a slip wall
-__device__ __forceinline__ long long neighbour(const Mesh& m, int ex, int ey, int ez, int d, int side) {
+// neighbour across face (d, side) or -1 for a slip wall (element indices are below 2^31)
+__device__ __forceinline__ int neighbour(const Mesh& m, int ex, int ey, int ez, int d, int side) {
     int c0 = ex, c1 = ey, c2 = ez;
     if (d == 0) {
         c0 += side ? 1 : -1;
@@ -211,7 +211,7 @@ __device__ __forceinline__ long long neighbour(const Mesh& m, int ex, int ey, in
         c2 += side ? 1 : -1;
         c2 = c2 < 0 ? c2 + m.nz : (c2 >= m.nz ? c2 - m.nz : c2);
     }
-    return (long long)(c0 + m.nx * (c1 + m.ny * c2));
+    return c0 + m.nx * (c1 + m.ny * c2);
 }
 
 // ---- 4-wide loads / stores (16-byte aligned for float, 32-byte for double)
@@ -1359,7 +1359,8 @@ __device__ __forceinline__ void ld4once(const S* p, P* q) {
 // Per-element context of phase B: the element, its x-line and its neighbours.
 template <class C>
 struct BCtx {
-    long long e, nxm, nxp, nym, nyp, nzm, nzp;
+    long long e;
+    int nxm, nxp, nym, nyp, nzm, nzp;   // 32-bit: each record address is one wide multiply-add
     int l, lj, lk;
     C hx, hy, hz;
 };
@@ -1404,7 +1405,11 @@ __device__ __forceinline__ BVar<P, C> b_load(const PB& B, const BCtx<C>& x, int 
     using S = typename PB::S_t;
     const Mesh& m = B.m;
     const bool defer = (B.flags & kDeferRK) != 0;
-    const long long e = x.e, nxm = x.nxm, nxp = x.nxp, nym = x.nym, nyp = x.nyp, nzm = x.nzm, nzp = x.nzp;
+    const long long e = x.e;
+    const int nxm = x.nxm, nxp = x.nxp, nym = x.nym, nyp = x.nyp, nzm = x.nzm, nzp = x.nzp;
+    // the records of an element, at this variable
+    auto fi = [&](int nb, int dir) { return B.fi + (dir * NV + v) * NF + (size_t)(unsigned)nb * (3 * NV * NF); };
+    auto fvr = [&](int nb, int dir) { return B.fv + (dir * 4 + v - 1) * NF + (size_t)(unsigned)nb * (3 * 4 * NF); };
     const int l = x.l, lj = x.lj, lk = x.lk;
     const C hx = x.hx, hy = x.hy, hz = x.hz;
     BVar<P, C> d;
@@ -1412,42 +1417,41 @@ __device__ __forceinline__ BVar<P, C> b_load(const PB& B, const BCtx<C>& x, int 
     for (int i = 0; i < 4; ++i) d.acc[i] = (C)0;
     // plus faces: the plus neighbours' minus-face records F_I - 1/2 Fv
     {
-        const C f0 = ldf<COH>(B.fi + ((nxp * 3 + 0) * NV + v) * NF + l);
+        const C f0 = ldf<COH>(fi(nxp, 0) + l);
 #pragma unroll
         for (int i = 0; i < 4; ++i) d.acc[i] = fma(-B.jac[0] * B.tc.gR[i], f0, d.acc[i]);
     }
     if (nyp >= 0) {
         C w[4];
-        ld4once<COH, C, C>(B.fi + ((nyp * 3 + 1) * NV + v) * NF + 4 * lk, w);
+        ld4once<COH, C, C>(fi(nyp, 1) + 4 * lk, w);
         const C c = -B.jac[1] * B.tc.gR[lj];
 #pragma unroll
         for (int i = 0; i < 4; ++i) d.acc[i] = fma(c, w[i], d.acc[i]);
     }
     {
         C w[4];
-        ld4once<COH, C, C>(B.fi + ((nzp * 3 + 2) * NV + v) * NF + 4 * lj, w);
+        ld4once<COH, C, C>(fi(nzp, 2) + 4 * lj, w);
         const C c = -B.jac[2] * B.tc.gR[lk];
 #pragma unroll
         for (int i = 0; i < 4; ++i) d.acc[i] = fma(c, w[i], d.acc[i]);
     }
     if (v > 0) {
         // minus faces: the minus neighbours' viscous fluxes at their plus faces
-        const int q = v - 1;
         {
-            const C a0 = ldf<COH>(B.fv + ((nxm * 3 + 0) * 4 + q) * NF + l);
+            const C a0 = ldf<COH>(fvr(nxm, 0) + l);
 #pragma unroll
             for (int i = 0; i < 4; ++i) d.acc[i] = fma(hx * B.tc.gL[i], a0, d.acc[i]);
         }
         if (nym >= 0) {
             C w[4];
-            ld4once<COH, C, C>(B.fv + ((nym * 3 + 1) * 4 + q) * NF + 4 * lk, w);
+            ld4once<COH, C, C>(fvr(nym, 1) + 4 * lk, w);
             const C c = hy * B.tc.gL[lj];
 #pragma unroll
             for (int i = 0; i < 4; ++i) d.acc[i] = fma(c, w[i], d.acc[i]);
         }
         {
             C w[4];
-            ld4once<COH, C, C>(B.fv + ((nzm * 3 + 2) * 4 + q) * NF + 4 * lj, w);
+            ld4once<COH, C, C>(fvr(nzm, 2) + 4 * lj, w);
             const C c = hz * B.tc.gL[lk];
 #pragma unroll
             for (int i = 0; i < 4; ++i) d.acc[i] = fma(c, w[i], d.acc[i]);
