@@ -141,7 +141,7 @@ struct od_ctx {
     // step. (Slabs exchange f64 layers and od_rhs_noalloc has no buffers: those
     // keep f64 storage.)
     bool narrow = false, wide_valid = false;
-    double* wide = nullptr;
+    double* wide = nullptr;   // first part of one allocation with U
     size_t state_bytes = 0;
     size_t elem_size = 4;
     long long nelem = 0;
@@ -545,15 +545,16 @@ static int create_ctx(const od_params* p, bool slab, od_ctx** out) {
         *out = c;
         return cuda_fail(c, e, "kernel attributes");
     }
-    for (int b = 0; b < 3; ++b) {
-        e = cudaMalloc(&c->U[b], c->buf_bytes);
+    if (c->narrow) {
+        e = cudaMalloc((void**)&c->wide, c->state_bytes + 3 * c->buf_bytes);
         if (e != cudaSuccess) {
             *out = c;
             return cuda_fail(c, e, "cudaMalloc state");
         }
+        for (int b = 0; b < 3; ++b) c->U[b] = (char*)c->wide + c->state_bytes + b * c->buf_bytes;
     }
-    if (c->narrow) {
-        e = cudaMalloc((void**)&c->wide, c->state_bytes);
+    for (int b = 0; b < 3 && !c->narrow; ++b) {
+        e = cudaMalloc(&c->U[b], c->buf_bytes);
         if (e != cudaSuccess) {
             *out = c;
             return cuda_fail(c, e, "cudaMalloc state");
@@ -595,7 +596,7 @@ void od_destroy(od_ctx* c) {
     for (auto ev : c->slab_ev) cudaEventDestroy(ev);
     for (auto ev : c->ev_halo)
         if (ev) cudaEventDestroy(ev);
-    for (int b = 0; b < 3; ++b)
+    for (int b = 0; b < 3 && !c->narrow; ++b)
         if (c->U[b]) cudaFree(c->U[b]);
     if (c->fv) cudaFree(c->fv);
     if (c->rhs) cudaFree(c->rhs);
