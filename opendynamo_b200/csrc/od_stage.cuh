@@ -26,13 +26,18 @@
 //        F_I - 1/2 Fv_own at the minus faces (all the minus neighbour still
 //        needs at its plus face), Fv_own at the plus faces
 //   P6  x-threads: pointwise Euler - viscous fluxes of their 4 points
-//        (rhs.cu:229-266); F_y, F_z -> smem, the x-divergence of the
-//        thread's own x-line accumulated in registers
-//   P7  x-threads: divergence of F_y / F_z at their 4 points from the
-//        x-lines of their k-plane / j-column (128-bit loads)
-//   P8  x-threads: RHS = -div + forcing (rhs.cu:505-509), lifting
-//        -(j_L g_L' + j_R g_R') jac (rk.cu:12-25), RK combination
+//        (rhs.cu:229-266), two at a time in packed arithmetic in the all-f32
+//        kernels; F_y, F_z -> smem, the x-divergence of the thread's own
+//        x-line accumulated in registers
+//   P7  divergence of F_y / F_z and the lifting -(j_L g_L' + j_R g_R') jac
+//        (rk.cu:12-25) of the faces: the thread's own y-line, then z-line, then
+//        x-line, the partial updates handed on through smem (kLineUpdate); the
+//        pipelines with f32 fluxes under an f64 state instead update a whole
+//        x-line from the x-lines of its k-plane and j-column
+//   P8  x-threads: RHS + forcing (rhs.cu:505-509), RK combination
 //        a*u0 + b*u + c*(RHS + lift) (rk.cu:27-83), 128-bit stores.
+//   An element's 16 threads are half of a warp: the passes are separated by
+//   warp barriers only.
 //   The face correction of the reference, j = F_I - 1/2(Fv_L + Fv_R) -
 //   (Fe_own - Fv_own), is then complete except for the terms that belong to
 //   the neighbour: F_I at the plus faces and -1/2 Fv_nbr at every non-wall
