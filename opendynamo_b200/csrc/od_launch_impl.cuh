@@ -38,6 +38,13 @@ constexpr bool has_feat_variant() {
 // 16, 1.09x at 24, 1.04x at 32, 1.5% at 40, 0.7% at 48; f64 1.24x at 4, 1.11x
 // at 8 to 16, 1.2% at 32, nothing at 48; but u64/c32 2% slower at 48 and 64.
 constexpr long long kDependentElems = 1 << 16;
+// Phase A that writes the closure's features: from 4096 elements only. Its own
+// dependent, the network, follows it into residence, and below that the
+// network's blocks poll beside phase B and phase A for longer than the launch
+// latency saves (20 steps with the closure, ordinary against dependent: 512
+// elements 2.34 against 2.51 ms, 1728 2.45 / 2.65, 2744 2.61 / 2.73; 4096 2.88 /
+// 2.82, 13824 5.04 / 4.94).
+constexpr long long kDependentFeatElems = 1 << 12;
 
 template <class S, class P, class C, class M, int FLUX, int EPB>
 cudaError_t launch_a(const StageAParams<S, P, C>& A, long long nelem, cudaStream_t s, bool feat = false) {
@@ -46,8 +53,8 @@ cudaError_t launch_a(const StageAParams<S, P, C>& A, long long nelem, cudaStream
     const size_t smem = sizeof(SlotFor<M, P, C>) * EPB;
     if constexpr (has_feat_variant<S, P, C, M>() && EPB == 4) {
         if (feat) {
-            return launch_dependent(nelem <= kDependentElems, stage_a_kernel<S, P, C, M, FLUX, EPB, true>, grid,
-                                    LPE * EPB, smem, s, A);
+            return launch_dependent(nelem >= kDependentFeatElems && nelem <= kDependentElems,
+                                    stage_a_kernel<S, P, C, M, FLUX, EPB, true>, grid, LPE * EPB, smem, s, A);
         }
     }
     if (feat) return cudaErrorInvalidValue;   // no variant writes the features for this launch
