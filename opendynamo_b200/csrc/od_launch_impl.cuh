@@ -38,6 +38,17 @@ constexpr bool has_feat_variant() {
 // 16, 1.09x at 24, 1.04x at 32, 1.5% at 40, 0.7% at 48; f64 1.24x at 4, 1.11x
 // at 8 to 16, 1.2% at 32, nothing at 48; but u64/c32 2% slower at 48 and 64.
 constexpr long long kDependentElems = 1 << 16;
+// Phase A with f32 fluxes is an ordinary launch at 1.7 to 4 blocks per SM: its
+// blocks then spread evenly, where a dependent's fill the gaps of phase B and
+// pile up on some SMs (10 steps, ordinary against dependent: f32 1100 elements
+// 384 / 426 us, 1728 382 / 397, 2197 445 / 475, but 700 378 / 352; u64/c32 424 /
+// 494, 442 / 457, 492 / 550; mixed 446 / 507, 504 / 457, 550 / 570; f64 is faster
+// as a dependent at all of these).
+template <class C>
+bool dependent_a(long long nelem, unsigned grid) {
+    return nelem <= kDependentElems && !(sizeof(C) == 4 && grid > 256 && grid <= 592);
+}
+
 // Phase A that writes the closure's features: from 4096 elements only. Its own
 // dependent, the network, follows it into residence, and below that the
 // network's blocks poll beside phase B and phase A for longer than the launch
@@ -58,7 +69,8 @@ cudaError_t launch_a(const StageAParams<S, P, C>& A, long long nelem, cudaStream
         }
     }
     if (feat) return cudaErrorInvalidValue;   // no variant writes the features for this launch
-    return launch_dependent(nelem <= kDependentElems, stage_a_kernel<S, P, C, M, FLUX, EPB>, grid, LPE * EPB, smem, s, A);
+    return launch_dependent(dependent_a<C>(nelem, grid), stage_a_kernel<S, P, C, M, FLUX, EPB>, grid, LPE * EPB, smem, s,
+                            A);
 }
 
 template <class S, class P, class C, class M, int FLUX>
