@@ -140,8 +140,13 @@ struct od_ctx {
     // view of the state: what was last set, or U[0] converted; valid until a
     // step. (Slabs exchange f64 layers and od_rhs_noalloc has no buffers: those
     // keep f64 storage.)
-    bool narrow = false, wide_valid = false;
-    double* wide = nullptr;   // first part of one allocation with U
+    // graphed: a step or a state copy has been captured on the stream. What a
+    // replay leaves is known on the device only, so from then on wide_word says
+    // there, in stream order, whether wide is the state; wide_valid keeps its
+    // value of that moment, which holds while the word is kWideAsBefore.
+    bool narrow = false, wide_valid = false, graphed = false;
+    double* wide = nullptr;        // first part of one allocation with U and wide_word
+    unsigned* wide_word = nullptr;
     size_t state_bytes = 0;
     size_t elem_size = 4;
     long long nelem = 0;
@@ -202,10 +207,15 @@ void set_jac(od_ctx* c, const od_params* p) {
     }
 }
 
+// od_ctx::wide_word: nothing written since the first capture; a state was set; a step was made
+constexpr unsigned kWideAsBefore = 0, kWideSet = 1;
+constexpr int kWideStaleByte = 2;
+
 // Conversions of a narrow context's state; vec: the f64 buffers are 16-byte
 // aligned. n is a multiple of 4; a value per step of 4 and thread.
 __global__ void __launch_bounds__(256) narrow_kernel(const double* __restrict__ src, double* __restrict__ copy,
-                                                     float* __restrict__ dst, size_t n, bool vec) {
+                                                     float* __restrict__ dst, size_t n, bool vec, unsigned* word) {
+    if (word && blockIdx.x == 0 && threadIdx.x == 0) *word = kWideSet;
     for (size_t i = 4 * ((size_t)blockIdx.x * 256 + threadIdx.x); i < n; i += 4 * (size_t)gridDim.x * 256) {
         double a[4];
         if (vec) {
@@ -222,15 +232,24 @@ __global__ void __launch_bounds__(256) narrow_kernel(const double* __restrict__ 
     }
 }
 
-__global__ void __launch_bounds__(256) widen_kernel(const float* __restrict__ src, double* __restrict__ dst, size_t n,
-                                                    bool vec) {
+// dst = src as f64, or, where word (null: no) says so, the exact values
+__global__ void __launch_bounds__(256) widen_kernel(const float* __restrict__ src, const double* exact,
+                                                    const unsigned* word, bool before, double* dst, size_t n, bool vec) {
+    const bool use = word && (*word == kWideAsBefore ? before : *word == kWideSet);
+    if (use && dst == exact) return;
     for (size_t i = 4 * ((size_t)blockIdx.x * 256 + threadIdx.x); i < n; i += 4 * (size_t)gridDim.x * 256) {
-        const float4 x = *reinterpret_cast<const float4*>(src + i);
-        if (vec) {
-            *reinterpret_cast<double2*>(dst + i) = make_double2(x.x, x.y);
-            *reinterpret_cast<double2*>(dst + i + 2) = make_double2(x.z, x.w);
+        double a[4];
+        if (use) {
+            for (int q = 0; q < 4; ++q) a[q] = exact[i + q];
         } else {
-            dst[i] = x.x; dst[i + 1] = x.y; dst[i + 2] = x.z; dst[i + 3] = x.w;
+            const float4 x = *reinterpret_cast<const float4*>(src + i);
+            a[0] = x.x; a[1] = x.y; a[2] = x.z; a[3] = x.w;
+        }
+        if (vec) {
+            *reinterpret_cast<double2*>(dst + i) = make_double2(a[0], a[1]);
+            *reinterpret_cast<double2*>(dst + i + 2) = make_double2(a[2], a[3]);
+        } else {
+            for (int q = 0; q < 4; ++q) dst[i + q] = a[q];
         }
     }
 }
@@ -238,20 +257,45 @@ __global__ void __launch_bounds__(256) widen_kernel(const float* __restrict__ sr
 unsigned convert_blocks(size_t n) { return (unsigned)std::min<size_t>((n / 4 + 255) / 256, 148 * 16); }
 bool aligned16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15) == 0; }
 
+// whether the device decides if wide is the state (od_ctx::graphed)
+bool by_word(od_ctx* c) {
+    cudaStreamCaptureStatus st = cudaStreamCaptureStatusNone;
+    if (!c->graphed && cudaStreamIsCapturing(c->stream, &st) == cudaSuccess && st != cudaStreamCaptureStatusNone)
+        c->graphed = true;
+    return c->graphed;
+}
+
 // src (f64, device) becomes the state of a narrow context
 cudaError_t narrow_state(od_ctx* c, const double* src) {
     const size_t n = c->state_bytes / 8;
+    const bool word = by_word(c);
     narrow_kernel<<<convert_blocks(n), 256, 0, c->stream>>>(src, src == c->wide ? nullptr : c->wide, (float*)c->U[0], n,
-                                                            aligned16(src));
-    c->wide_valid = true;
+                                                            aligned16(src), word ? c->wide_word : nullptr);
+    if (!word) c->wide_valid = true;
     return cudaGetLastError();
 }
 
 // an f32 buffer of a narrow context as f64
 cudaError_t widen(od_ctx* c, const void* src, double* dst) {
     const size_t n = c->state_bytes / 8;
-    widen_kernel<<<convert_blocks(n), 256, 0, c->stream>>>((const float*)src, dst, n, aligned16(dst));
+    widen_kernel<<<convert_blocks(n), 256, 0, c->stream>>>((const float*)src, nullptr, nullptr, false, dst, n,
+                                                           aligned16(dst));
     return cudaGetLastError();
+}
+
+// the state of a graphed narrow context as f64 (into wide: what is not there already)
+cudaError_t widen_by_word(od_ctx* c, double* dst) {
+    const size_t n = c->state_bytes / 8;
+    widen_kernel<<<convert_blocks(n), 256, 0, c->stream>>>((const float*)c->U[0], c->wide, c->wide_word, c->wide_valid,
+                                                           dst, n, aligned16(dst));
+    return cudaGetLastError();
+}
+
+// a step is about to change the state of a narrow context
+cudaError_t wide_stale(od_ctx* c) {
+    if (by_word(c)) return cudaMemsetAsync(c->wide_word, kWideStaleByte, sizeof(unsigned), c->stream);
+    c->wide_valid = false;
+    return cudaSuccess;
 }
 
 cudaError_t copy_narrow(od_ctx* c, void* other, bool to_ctx, cudaMemcpyKind kind) {
@@ -260,7 +304,11 @@ cudaError_t copy_narrow(od_ctx* c, void* other, bool to_ctx, cudaMemcpyKind kind
         cudaError_t e = cudaMemcpyAsync(c->wide, other, c->state_bytes, kind, c->stream);
         return e == cudaSuccess ? narrow_state(c, c->wide) : e;
     }
-    if (!c->wide_valid) {
+    if (by_word(c)) {
+        if (kind == cudaMemcpyDeviceToDevice) return widen_by_word(c, (double*)other);
+        cudaError_t e = widen_by_word(c, c->wide);
+        if (e != cudaSuccess) return e;
+    } else if (!c->wide_valid) {
         if (kind == cudaMemcpyDeviceToDevice) return widen(c, c->U[0], (double*)other);
         cudaError_t e = widen(c, c->U[0], c->wide);
         if (e != cudaSuccess) return e;
@@ -546,7 +594,11 @@ static int create_ctx(const od_params* p, bool slab, od_ctx** out) {
         return cuda_fail(c, e, "kernel attributes");
     }
     if (c->narrow) {
-        e = cudaMalloc((void**)&c->wide, c->state_bytes + 3 * c->buf_bytes);
+        e = cudaMalloc((void**)&c->wide, c->state_bytes + 3 * c->buf_bytes + sizeof(unsigned));
+        if (e == cudaSuccess) {
+            c->wide_word = (unsigned*)((char*)c->wide + c->state_bytes + 3 * c->buf_bytes);
+            e = cudaMemsetAsync(c->wide_word, 0, sizeof(unsigned), c->stream);
+        }
         if (e != cudaSuccess) {
             *out = c;
             return cuda_fail(c, e, "cudaMalloc state");
@@ -741,7 +793,10 @@ int od_step(od_ctx* c, int n_steps, double dt) {
     if (!c->have_state) return fail(c, OD_ERR_STATE, "no state set");
     if (c->slab) return fail(c, OD_ERR_STATE, "a slab context steps through od_slab_stage");
     if (int rc = set_device(c)) return rc;
-    if (n_steps > 0) c->wide_valid = false;
+    if (n_steps > 0 && c->narrow) {
+        const cudaError_t e = wide_stale(c);
+        if (e != cudaSuccess) return cuda_fail(c, e, "state view");
+    }
     for (int s = 0; s < n_steps; ++s)
         for (int k = 0; k < 3; ++k) {
             const RkStage r = rk_stage(c, k, dt);
@@ -997,10 +1052,14 @@ int od_diagnostics(od_ctx* c, double* vol6, double* prof, size_t prof_len) {
         c->diag = d;
     }
     e = cudaMemsetAsync(d, 0, bytes, c->stream);
+    bool wide = c->narrow && c->wide_valid;
+    if (e == cudaSuccess && c->narrow && by_word(c)) {
+        e = widen_by_word(c, c->wide);
+        wide = true;
+    }
     if (e == cudaSuccess)
-        e = od::launch_diag(c->narrow && c->wide_valid ? (const void*)c->wide : c->U[0],
-                            c->narrow ? c->wide_valid : c->elem_size == 8, c->p.nx, c->p.ny, c->p.nz, c->p.lx, c->p.ly, c->p.lz,
-                            c->tab, d, prof ? d + 6 : nullptr, c->stream);
+        e = od::launch_diag(wide ? (const void*)c->wide : c->U[0], c->narrow ? wide : c->elem_size == 8, c->p.nx,
+                            c->p.ny, c->p.nz, c->p.lx, c->p.ly, c->p.lz, c->tab, d, prof ? d + 6 : nullptr, c->stream);
     std::vector<double> h(6 + nprof);
     if (e == cudaSuccess) e = cudaMemcpyAsync(h.data(), d, bytes, cudaMemcpyDeviceToHost, c->stream);
     if (e == cudaSuccess) e = cudaStreamSynchronize(c->stream);
