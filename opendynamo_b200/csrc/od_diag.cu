@@ -93,7 +93,13 @@ __global__ void __launch_bounds__(32 * kDiagWarps, 3) diag_kernel(const S* __res
         const S* p = u + ((long long)ex + (long long)nx * (ey + (long long)P.ny * ez)) * 64 + 4 * l;
         double s[5][4];
 #pragma unroll
-        for (int v = 0; v < 5; ++v) load_line(p + v * npts, s[v]);
+        for (int v = 0; v < 5; ++v) {
+            load_line(p + v * npts, s[v]);
+            // no partner: a state whose zero weight gives zero (the first
+            // element's infinite or NaN values times zero would not)
+#pragma unroll
+            for (int i = 0; i < 4; ++i) s[v][i] = live ? s[v][i] : (v == 0 ? 1.0 : 0.0);
+        }
         __syncwarp();   // the pass before is done with the planes
 #pragma unroll
         for (int v = 0; v < 4; ++v) {
