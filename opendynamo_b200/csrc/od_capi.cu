@@ -298,18 +298,32 @@ cudaError_t wide_stale(od_ctx* c) {
     return cudaSuccess;
 }
 
+// whether the conversion kernels may use p: f64-aligned memory of the context's
+// GPU. Other addresses (any alignment, another GPU's memory with or without
+// peer access, managed memory) go through a copy, which takes them all.
+bool kernel_address(od_ctx* c, const void* p) {
+    if (reinterpret_cast<uintptr_t>(p) & (sizeof(double) - 1)) return false;
+    cudaPointerAttributes a{};
+    if (cudaPointerGetAttributes(&a, p) != cudaSuccess) {
+        (void)cudaGetLastError();
+        return false;
+    }
+    return a.type == cudaMemoryTypeDevice && a.device == c->p.device;
+}
+
 cudaError_t copy_narrow(od_ctx* c, void* other, bool to_ctx, cudaMemcpyKind kind) {
+    const bool direct = kind == cudaMemcpyDeviceToDevice && kernel_address(c, other);
     if (to_ctx) {
-        if (kind == cudaMemcpyDeviceToDevice) return narrow_state(c, (const double*)other);
+        if (direct) return narrow_state(c, (const double*)other);
         cudaError_t e = cudaMemcpyAsync(c->wide, other, c->state_bytes, kind, c->stream);
         return e == cudaSuccess ? narrow_state(c, c->wide) : e;
     }
     if (by_word(c)) {
-        if (kind == cudaMemcpyDeviceToDevice) return widen_by_word(c, (double*)other);
+        if (direct) return widen_by_word(c, (double*)other);
         cudaError_t e = widen_by_word(c, c->wide);
         if (e != cudaSuccess) return e;
     } else if (!c->wide_valid) {
-        if (kind == cudaMemcpyDeviceToDevice) return widen(c, c->U[0], (double*)other);
+        if (direct) return widen(c, c->U[0], (double*)other);
         cudaError_t e = widen(c, c->U[0], c->wide);
         if (e != cudaSuccess) return e;
         c->wide_valid = true;
