@@ -20,27 +20,8 @@ namespace od {
 
 enum Flux : int { kSlau2 = 0, kAusmPlus = 1, kRusanov = 2 };
 
-// 1/x in f64 from an estimate r of relative error below 2^-19: one step of the
-// third-order iteration r (1 + e + e^2), e = 1 - r x (Householder's method for
-// f(r) = 1/r - x), error e^3 before the one rounding of the result.
-__device__ __forceinline__ double rcp_refined(double x, double r) {
-    const double e = fma(-x, r, 1.0);
-    return fma(r, fma(e, e, e), r);
-}
-
-// 1/x in f64 for |x| in the normal range, within 0.56 ulp (rcp.approx.ftz.f64:
-// 20 mantissa bits); NaN for zero, infinite and subnormal x. Four operations;
-// the f64 division is a chain of about ten and a branch.
-__device__ __forceinline__ double rcp_f64(double x) {
-    double r;
-    asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(r) : "d"(x));
-    return rcp_refined(x, r);
-}
-
 // Division / reciprocal / square root policy. MathIeee: correctly rounded
-// (the reference with fast_math = false) but for the f64 reciprocal and
-// division, which are within an ulp (40^3 f64 step 1.46 -> 1.38 ms; error of a
-// step against float64 unchanged).
+// (the reference with fast_math = false, and every f64 operation).
 // MathFast: for f32 operands the approximate PTX forms (rcp.approx,
 // sqrt.approx, ~1-2 ulp), the arithmetic of the reference's default
 // --use_fast_math build; f64 operands stay IEEE (fast math does not touch them).
@@ -48,20 +29,9 @@ struct MathIeee {
     static constexpr bool kSutherland = false;
     static constexpr bool kWideState = false;
     template <class T>
-    static __device__ __forceinline__ T rcp(T x) {
-        if constexpr (sizeof(T) == 8) return rcp_f64(x);
-        else return (T)1.0 / x;
-    }
+    static __device__ __forceinline__ T rcp(T x) { return (T)1.0 / x; }
     template <class T>
-    static __device__ __forceinline__ T div(T a, T b) {
-        if constexpr (sizeof(T) == 8) {
-            // the quotient corrected by its remainder
-            const T r = rcp_f64(b), q = a * r;
-            return fma(fma(-b, q, a), r, q);
-        } else {
-            return a / b;
-        }
-    }
+    static __device__ __forceinline__ T div(T a, T b) { return a / b; }
     template <class T>
     static __device__ __forceinline__ T sqrt(T x) { return ::sqrt(x); }
 };
@@ -149,6 +119,16 @@ struct FaceState {
     C p;      // praw clamped (the inviscid fluxes and sound speeds)
 };
 
+// 1/x in f64 from an f32 estimate r0 of it (rcp.approx: relative error below
+// 2^-22): one step of the third-order iteration r0 (1 + e + e^2), e = 1 - r0 x
+// (Householder's method for f(r) = 1/r - x), error e^3 below 2^-66 before
+// rounding. x in the f32 range.
+__device__ __forceinline__ double rcp_refined(double x, float r0) {
+    const double r = (double)r0;
+    const double e = fma(-x, r, 1.0);
+    return fma(r, fma(e, e, e), r);
+}
+
 // kWideState: the pressure recovered in the state arithmetic's precision P
 // (f64 in the mixed form, whose f64 division of the kinetic energy, 17 of them
 // a thread, is a product with the refined reciprocal: 96^3 step 14.9 -> 14.2 ms).
@@ -162,7 +142,7 @@ __device__ __forceinline__ FaceState<C> make_face_state(const P* qp) {
     s.ir = M::rcp(s.q[0]);
     if constexpr (M::kWideState) {
         if constexpr (sizeof(P) == 8) {
-            const P ke = ((P)0.5 * (qp[1] * qp[1] + qp[2] * qp[2] + qp[3] * qp[3])) * rcp_refined(qp[0], (double)s.ir);
+            const P ke = ((P)0.5 * (qp[1] * qp[1] + qp[2] * qp[2] + qp[3] * qp[3])) * rcp_refined(qp[0], s.ir);
             s.praw = (C)(Gas<P>::gm1() * (qp[4] - ke));
         } else {
             s.praw = raw_pressure<M, P>(qp[0], qp[1], qp[2], qp[3], qp[4]);
