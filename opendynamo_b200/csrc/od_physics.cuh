@@ -265,16 +265,18 @@ __device__ __forceinline__ VolumeFluxes<C> volume_fluxes(const FaceState<C>& s, 
     const C t01 = mi * (w(0, 1) + w(1, 0)), t02 = mi * (w(0, 2) + w(2, 0)), t12 = mi * (w(1, 2) + w(2, 1));
     const C u = s.vel[0], v = s.vel[1], x = s.vel[2];
     VolumeFluxes<C> f;
-    f.m00 = s.q[1] * u - t00 + s.p;
-    f.m11 = s.q[2] * v - t11 + s.p;
-    f.m22 = s.q[3] * x - t22 + s.p;
+    f.m00 = s.q[1] * u + s.p - t00;
+    f.m11 = s.q[2] * v + s.p - t11;
+    f.m22 = s.q[3] * x + s.p - t22;
     f.m01 = s.q[1] * v - t01;
     f.m02 = s.q[1] * x - t02;
     f.m12 = s.q[2] * x - t12;
     const C h = s.q[4] + s.p, ce = (s.ke - s.ein) * s.ir, k = mi * gamma_over_pr<C>();
-    f.e[0] = h * u - k * heat_bracket(s, g, ce, 0) - u * t00 - v * t01 - x * t02;
-    f.e[1] = h * v - k * heat_bracket(s, g, ce, 1) - u * t01 - v * t11 - x * t12;
-    f.e[2] = h * x - k * heat_bracket(s, g, ce, 2) - u * t02 - v * t12 - x * t22;
+    // the viscous terms first: h u is orders of magnitude above them, and every
+    // term added to it would round at its size
+    f.e[0] = h * u - (k * heat_bracket(s, g, ce, 0) + u * t00 + v * t01 + x * t02);
+    f.e[1] = h * v - (k * heat_bracket(s, g, ce, 1) + u * t01 + v * t11 + x * t12);
+    f.e[2] = h * x - (k * heat_bracket(s, g, ce, 2) + u * t02 + v * t12 + x * t22);
     return f;
 }
 
@@ -341,11 +343,11 @@ __device__ __forceinline__ VolumeFluxes2 volume_fluxes2(QF q, GF g, float mu0, f
     f.m12 = fma2(q2, x, t12);
     const F2 nk = nmi * F2(gamma_over_pr<float>());
     const F2 b0 = fma2(nx, a20, fma2(nv, a10, fma2(nu, a00, fma2(ce, r0, g(12)))));
-    f.e[0] = fma2(nk, b0, fma2(x, t02, fma2(v, t01, fma2(u, t00, h * u))));
+    f.e[0] = fma2(h, u, fma2(x, t02, fma2(v, t01, fma2(u, t00, nk * b0))));
     const F2 b1 = fma2(nx, a21, fma2(nv, a11, fma2(nu, a01, fma2(ce, r1, g(13)))));
-    f.e[1] = fma2(nk, b1, fma2(x, t12, fma2(v, t11, fma2(u, t01, h * v))));
+    f.e[1] = fma2(h, v, fma2(x, t12, fma2(v, t11, fma2(u, t01, nk * b1))));
     const F2 b2 = fma2(nx, a22, fma2(nv, a12, fma2(nu, a02, fma2(ce, r2, g(14)))));
-    f.e[2] = fma2(nk, b2, fma2(x, t22, fma2(v, t12, fma2(u, t02, h * x))));
+    f.e[2] = fma2(h, x, fma2(x, t22, fma2(v, t12, fma2(u, t02, nk * b2))));
     return f;
 }
 
