@@ -461,8 +461,8 @@ __global__ void __launch_bounds__(256) gather_kernel(const bf16* __restrict__ Xp
 // fp32 rows [M x 384], or (POOL) rows of the bf16 target pool [n x 320].
 // Block (x, y): 64 rows, 64 columns.
 template <bool POOL, bool VEC>
-__global__ void __launch_bounds__(256) loss_grad_kernel(const float* __restrict__ Y, const float* __restrict__ T,
-                                                        const bf16* __restrict__ Tp, const long long* __restrict__ rows,
+__global__ void __launch_bounds__(256) loss_grad_kernel(const float* Y, const float* T, const bf16* __restrict__ Tp,
+                                                        const long long* __restrict__ rows,
                                                         int M, int mv, float g, bf16* __restrict__ dY,
                                                         bf16* __restrict__ dYT, double* loss) {
     od::dependent_start();
@@ -479,7 +479,7 @@ __global__ void __launch_bounds__(256) loss_grad_kernel(const float* __restrict_
             float y[8], t[8];
 #pragma unroll
             for (int h = 0; h < 2; ++h)
-                *reinterpret_cast<float4*>(y + 4 * h) = __ldg(reinterpret_cast<const float4*>(Y + at) + h);
+                *reinterpret_cast<float4*>(y + 4 * h) = reinterpret_cast<const float4*>(Y + at)[h];
             if constexpr (POOL) {
                 const uint4 w = pool8<VEC>(Tp + rows[m] * kOut + n0 + c);
                 const uint32_t u[4] = {w.x, w.y, w.z, w.w};
@@ -491,7 +491,7 @@ __global__ void __launch_bounds__(256) loss_grad_kernel(const float* __restrict_
             } else {
 #pragma unroll
                 for (int h = 0; h < 2; ++h)
-                    *reinterpret_cast<float4*>(t + 4 * h) = __ldg(reinterpret_cast<const float4*>(T + at) + h);
+                    *reinterpret_cast<float4*>(t + 4 * h) = reinterpret_cast<const float4*>(T + at)[h];
             }
             bf16 b[8];
 #pragma unroll
@@ -551,7 +551,7 @@ __device__ __forceinline__ float row_sum(const bf16* AT, int M, int n, int lane)
     float s[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
 #pragma unroll 8
     for (int q = lane; q < M / 8; q += 32) {
-        const uint4 w = __ldg(row + q);
+        const uint4 w = row[q];
         const uint32_t u[4] = {w.x, w.y, w.z, w.w};
 #pragma unroll
         for (int i = 0; i < 4; ++i) {

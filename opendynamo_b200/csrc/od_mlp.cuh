@@ -423,7 +423,7 @@ __device__ __forceinline__ void gemm_tile(const GemmArgs& g, int bx, int by, int
                 for (int it = 0; it < 8; ++it) {
                     const int rr = 4 * it + (lane >> 3), q = lane & 7;
                     *stage_f32_at(stg, rr, q) =
-                        __ldg(reinterpret_cast<const float4*>(g.z_in + (size_t)(row0 + rr) * g.N + n + 4 * q));
+                        *reinterpret_cast<const float4*>(g.z_in + (size_t)(row0 + rr) * g.N + n + 4 * q);
                 }
                 __syncwarp();
 #pragma unroll
