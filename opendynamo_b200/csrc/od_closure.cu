@@ -705,7 +705,10 @@ struct od_mlp {
     long long off_w[4], off_b[4];
     int rows[4], cols[4];
     bf16 *wb[4] = {}, *wbT[4] = {};
-    bf16* wt = nullptr;   // the fused inference kernel's weight image (refreshed with wb)
+    // the fused inference kernel's weight image (refreshed with wb). That kernel
+    // reads it and the biases in w before it waits for the kernels ahead of it on
+    // its stream: whatever writes them is complete before the writing call returns
+    bf16* wt = nullptr;
     // activations
     float* Z[3] = {};
     bf16 *A[3] = {}, *AT[3] = {};

@@ -238,10 +238,14 @@ __device__ __forceinline__ bool fused_failed(FusedSmem& sm) { return *(volatile 
 // MMAs are complete (its `bar` commit).
 __device__ __forceinline__ void fused_loader(const FusedArgs& g, FusedSmem& sm) {
     int issued = 0;
-    // The weights and biases do not depend on the kernel launched before this
-    // one (phase A or the features kernel, which may let this kernel start
-    // early): the first weight tiles are requested before waiting for it, the
-    // features after.
+    // The first weight tiles are requested (and the biases read) before waiting
+    // for the kernel launched before this one (phase A or the features kernel,
+    // which may let this kernel start early), the features after. That kernel,
+    // and with phase A a dependent itself also those before it, may then still
+    // run, so no kernel in flight may be writing the weights: every call that
+    // writes them (od_mlp_set_params, od_mlp_train_step) waits for its stream
+    // before it returns. A call that left them to the device would have to
+    // move these reads behind the wait.
     for (int i = 0; i < kFStages; ++i) {
         fused_load(g, sm, i, blockIdx.x, false);
         ++issued;

@@ -80,3 +80,20 @@ def test_row_sums_read_coherently():
     text = _sources()["od_closure.cu"]
     i = text.index("float row_sum(")
     assert "__ldg" not in _balanced(text, text.index("{", i), "{}")
+
+
+def test_weights_are_complete_when_the_call_that_writes_them_returns():
+    """(The inference kernel reads them before griddepcontrol.wait.)"""
+    text = _sources()["od_closure.cu"]
+    writers = set()
+    for m in re.finditer(r"\bint (od_mlp_\w+)\(", text):
+        params = _balanced(text, m.end() - 1, "()")
+        i = m.end() - 1 + len(params)
+        if text[i:i + 2] == ";\n":
+            continue
+        body = _balanced(text, text.index("{", i), "{}")
+        if re.search(r"cast_weights_kernel|adam_kernel|tile_fused_weights|cudaMemcpyAsync\(m->w\b", body):
+            writers.add(m.group(1))
+            last = max(body.rfind("cudaStreamSynchronize(m->stream)"), body.rfind("read_status(m"))
+            assert last > max(body.rfind(k) for k in ("cast_weights_kernel", "adam_kernel", "tile_fused_weights")), m.group(1)
+    assert writers == {"od_mlp_set_params", "od_mlp_train_step"}
