@@ -38,15 +38,26 @@ constexpr bool has_feat_variant() {
 // 16, 1.09x at 24, 1.04x at 32, 1.5% at 40, 0.7% at 48; f64 1.24x at 4, 1.11x
 // at 8 to 16, 1.2% at 32, nothing at 48; but u64/c32 2% slower at 48 and 64.
 constexpr long long kDependentElems = 1 << 16;
-// Phase A with f32 fluxes is an ordinary launch at 1.7 to 4 blocks per SM: its
-// blocks then spread evenly, where a dependent's fill the gaps of phase B and
-// pile up on some SMs (10 steps, ordinary against dependent: f32 1100 elements
-// 384 / 426 us, 1728 382 / 397, 2197 445 / 475, but 700 378 / 352; u64/c32 424 /
-// 494, 442 / 457, 492 / 550; mixed 446 / 507, 504 / 457, 550 / 570; f64 is faster
-// as a dependent at all of these).
-template <class C>
-bool dependent_a(long long nelem, unsigned grid) {
-    return nelem <= kDependentElems && !(sizeof(C) == 4 && grid > 256 && grid <= 592);
+// Phase A with f32 fluxes is an ordinary launch on meshes that give an SM some
+// of its places only: its blocks then spread evenly, where a dependent's fill
+// the gaps that phase B's leave and pile up on some SMs. The band is in elements
+// (blocks of 2 and of 4 elements behave alike). 10 steps, dependent / ordinary,
+// geometric means over random meshes of the range (elements: ratio):
+//   f32     384-511: 0.95  512-639: 0.97 | 640-767: 1.04  768-1023: 1.06
+//           1024-1791: 1.11  1792-2047: 0.91  2048-3071: 1.07
+//           3072-3399: 1.03 | 3584-4095: 0.89
+//   u64/c32 256-383: 0.90 | 384-511: 1.06  512-767: 1.10  768-1791: 1.15
+//           1792-2047: 0.93  2048-3071: 1.11  3072-3399: 1.06 | 3584-4095: 0.92
+//   mixed   256-383: 0.96 | 384-511: 1.02  512-767: 1.14  768-1535: 1.12
+//           1536-1791: 0.90  1792-2047: 1.13  2048-2559: 1.04 | 2560-3583: 0.92
+// Single meshes scatter by 0.8 to 1.25 inside it. f64 fluxes gain as dependents
+// nearly everywhere (0.89 to 0.97; 640-1023: 1.04).
+template <class P, class C, class M>
+bool dependent_a(long long nelem) {
+    if (nelem > kDependentElems) return false;
+    if (sizeof(C) == 8) return true;
+    const long long lo = M::kWideState ? 384 : 640, hi = sizeof(P) == 8 ? 2560 : 3400;
+    return nelem < lo || nelem >= hi;
 }
 
 // Phase A that writes the closure's features: from 4096 elements only. Its own
@@ -69,7 +80,7 @@ cudaError_t launch_a(const StageAParams<S, P, C>& A, long long nelem, cudaStream
         }
     }
     if (feat) return cudaErrorInvalidValue;   // no variant writes the features for this launch
-    return launch_dependent(dependent_a<C>(nelem, grid), stage_a_kernel<S, P, C, M, FLUX, EPB>, grid, LPE * EPB, smem, s,
+    return launch_dependent(dependent_a<P, C, M>(nelem), stage_a_kernel<S, P, C, M, FLUX, EPB>, grid, LPE * EPB, smem, s,
                             A);
 }
 
