@@ -904,18 +904,15 @@ __device__ __forceinline__ void face_grad_pass(const PA& A, Slot& sm, long long 
 
 // Rows of the dead gradient that hold F_y and F_z between P6 and P7. F_y of
 // rho w is F_z of rho v, and the mass fluxes are the momenta, read from the
-// state (kWideState: all ten fluxes in rows 0-9).
+// state. (kWideState: all ten fluxes, F_y in rows 0-4 and F_z in rows 5-9.)
 constexpr int kFy1 = 0, kFy2 = 1, kFy3 = 2, kFy4 = 3, kFz1 = 4, kFz2 = kFy3, kFz3 = 5, kFz4 = 6;
 
-template <class M, int D, class Slot>
+template <int D, class Slot>
 __device__ __forceinline__ const auto* flux_row(const Slot& sm, int v) {
-    if constexpr (M::kWideState) {
-        return &sm.g[(D == 1 ? 0 : 5) + v][0];
-    } else if constexpr (D == 1) {
+    if constexpr (D == 1)
         return v == 0 ? &sm.u[2][0] : &sm.g[v == 1 ? kFy1 : v == 2 ? kFy2 : v == 3 ? kFy3 : kFy4][0];
-    } else {
+    else
         return v == 0 ? &sm.u[3][0] : &sm.g[v == 1 ? kFz1 : v == 2 ? kFz2 : v == 3 ? kFz3 : kFz4][0];
-    }
 }
 
 // RK combination a*u0 + b*u + c*R of variable v on the x-line, or (deferred
@@ -958,56 +955,37 @@ __device__ __forceinline__ void store_update(const PA& A, const Slot& sm, int x,
 template <class M, class PA, class Slot, class P = typename PA::P_t, class C = typename PA::C_t>
 __device__ __forceinline__ void stage_a_update(const PA& A, Slot& sm, long long ec, int l, int swz,
                                                const C (&divx)[NV][4], const C (&jx)[2][NV]) {
+    static_assert(M::kWideState && sizeof(C) == 4, "every other pipeline updates by lines");
     const int lj = l & 3, lk = l >> 2;   // this x-line's (j, k)
-    C cy[4], cz[4];   // derivative rows of this thread's j (y) and k (z); not kWideState: negated
+    C cy[4], cz[4];   // derivative rows of this thread's j (y) and k (z)
 #pragma unroll
     for (int mm = 0; mm < 4; ++mm) {
-        cy[mm] = M::kWideState ? A.sc.d[1][lj * 4 + mm] : A.sc.nd[1][lj * 4 + mm];
-        cz[mm] = M::kWideState ? A.sc.d[2][lk * 4 + mm] : A.sc.nd[2][lk * 4 + mm];
+        cy[mm] = A.sc.d[1][lj * 4 + mm];
+        cz[mm] = A.sc.d[2][lk * 4 + mm];
     }
 #pragma unroll
     for (int v = 0; v < NV; ++v) {
-        C rt[4], jy0[4], jy1[4], jz0[4], jz1[4];
-        const C* fy = flux_row<M, 1>(sm, v);
-        const C* fz = flux_row<M, 2>(sm, v);
-        if constexpr (M::kWideState) {
-            C dy[4], dz[4];
+        C rt[4], dy[4], dz[4], jy0[4], jy1[4], jz0[4], jz1[4];
+        const C* fy = sm.g[v];
+        const C* fz = sm.g[5 + v];
 #pragma unroll
-            for (int mm = 0; mm < 4; ++mm) {
-                C f[4];
-                ld_xline(fy, sw<C>(4 * (mm + 4 * lk), swz), f);
+        for (int mm = 0; mm < 4; ++mm) {
+            C f[4];
+            ld_xline(fy, sw<C>(4 * (mm + 4 * lk), swz), f);
 #pragma unroll
-                for (int i = 0; i < 4; ++i) dy[i] = mm == 0 ? cy[0] * f[i] : fma(cy[mm], f[i], dy[i]);
-            }
+            for (int i = 0; i < 4; ++i) dy[i] = mm == 0 ? cy[0] * f[i] : fma(cy[mm], f[i], dy[i]);
+        }
 #pragma unroll
-            for (int mm = 0; mm < 4; ++mm) {
-                C f[4];
-                ld_xline(fz, sw<C>(4 * (lj + 4 * mm), swz), f);
+        for (int mm = 0; mm < 4; ++mm) {
+            C f[4];
+            ld_xline(fz, sw<C>(4 * (lj + 4 * mm), swz), f);
 #pragma unroll
-                for (int i = 0; i < 4; ++i) dz[i] = mm == 0 ? cz[0] * f[i] : fma(cz[mm], f[i], dz[i]);
-            }
+            for (int i = 0; i < 4; ++i) dz[i] = mm == 0 ? cz[0] * f[i] : fma(cz[mm], f[i], dz[i]);
+        }
 #pragma unroll
-            for (int i = 0; i < 4; ++i) {
-                rt[i] = -((divx[v][i] + dy[i]) + dz[i]);
-                if (v == 1) rt[i] += A.forcing;
-            }
-        } else {
-#pragma unroll
-            for (int i = 0; i < 4; ++i) rt[i] = divx[v][i];
-#pragma unroll
-            for (int mm = 0; mm < 4; ++mm) {
-                C f[4];
-                ld_xline(fy, sw<C>(4 * (mm + 4 * lk), swz), f);
-#pragma unroll
-                for (int i = 0; i < 4; ++i) rt[i] = fma(cy[mm], f[i], rt[i]);
-            }
-#pragma unroll
-            for (int mm = 0; mm < 4; ++mm) {
-                C f[4];
-                ld_xline(fz, sw<C>(4 * (lj + 4 * mm), swz), f);
-#pragma unroll
-                for (int i = 0; i < 4; ++i) rt[i] = fma(cz[mm], f[i], rt[i]);
-            }
+        for (int i = 0; i < 4; ++i) {
+            rt[i] = -((divx[v][i] + dy[i]) + dz[i]);
+            if (v == 1) rt[i] += A.forcing;
         }
         ld4s(&sm.j[0][v][4 * lk], jy0);
         ld4s(&sm.j[1][v][4 * lk], jy1);
@@ -1017,9 +995,6 @@ __device__ __forceinline__ void stage_a_update(const PA& A, Slot& sm, long long 
 #pragma unroll
         for (int i = 0; i < 4; ++i) {
             C r = rt[i];
-            if constexpr (sizeof(C) == 8) {
-                if (A.flags & kRoundRhs) r = (C)(float)r;
-            }
             // lifting -(j_L g_L' + j_R g_R') jac of the six faces (rk.cu:12-25)
             r = fma(jx0, A.sc.nl[0][i], r);
             r = fma(jx1, A.sc.nr[0][i], r);
@@ -1073,7 +1048,7 @@ __device__ __forceinline__ void update_pass(const PA& A, Slot& sm, const L& li, 
 #pragma unroll
     for (int v = 0; v < NV; ++v) {
         C f[4], r[4];
-        if constexpr (DIV) row_line_load<D>(flux_row<M, D>(sm, v), li, f);
+        if constexpr (DIV) row_line_load<D>(flux_row<D>(sm, v), li, f);
         if constexpr (!FRESH) row_line_load<D>(&sm.g[kR + v][0], li, r);
         line_terms<D, FRESH, DIV, LIFT>(A, f, j[0][v], j[1][v], r);
         row_line_store<D>(&sm.g[kR + v][0], li, r);

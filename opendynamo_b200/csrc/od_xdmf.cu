@@ -131,7 +131,7 @@ std::string fmt_g(const char* f, double x) {
 extern "C" int od_point_fields(const void* planes, int u_f64, int nx, int ny, int nz, float* out, void* stream) {
     if (!planes || !out || nx <= 0 || ny <= 0 || nz <= 0) return OD_ERR_ARG;
     const long long npts = 64LL * nx * ny * nz;
-    if (ny > 65535 || (nz + 7) / 8 > 65535) return OD_ERR_ARG;
+    if (ny > 65535 || (nz + 7) / 8 > 65535) return OD_ERR_ARG;   // mesh limits of this call
     const long long warps = (long long)nx * ny * ((nz + 7) / 8);
     const long long grid = (warps + od::kPfWarps - 1) / od::kPfWarps;
     if (grid > 0x7fffffffLL || (long long)nx * ny > 0xffffffffLL) return OD_ERR_ARG;
