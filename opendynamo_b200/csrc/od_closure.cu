@@ -836,8 +836,9 @@ constexpr size_t kStatusBytes = 16;   // loss and err, cleared and read back tog
 
 cudaError_t clear_status(od_mlp* m) { return cudaMemsetAsync(m->loss, 0, kStatusBytes, m->stream); }
 
-// waits for the stream; the loss sum of the calls since clear_status
-int read_status(od_mlp* m, double* loss) {
+// waits for the stream; loss (may be null; left alone when that fails): the
+// loss sum of the calls since clear_status over n
+int read_status(od_mlp* m, double* loss, double n = 1.0) {
     struct {
         double loss;
         int err, pad;
@@ -846,7 +847,7 @@ int read_status(od_mlp* m, double* loss) {
     cudaError_t e = cudaMemcpyAsync(&h, m->loss, sizeof h, cudaMemcpyDeviceToHost, m->stream);
     if (e == cudaSuccess) e = cudaStreamSynchronize(m->stream);
     if (e != cudaSuccess) return mfail(m, OD_ERR_CUDA, cudaGetErrorString(e));
-    if (loss) *loss = h.loss;
+    if (loss) *loss = h.loss / n;
     if (h.err) return mfail(m, OD_ERR_CUDA, "tensor-core GEMM wait timed out");
     return OD_OK;
 }
@@ -996,10 +997,7 @@ int od_mlp_gradients(od_mlp* m, const void* X, const void* XT, const float* T, i
     if (e == cudaSuccess && grads)
         e = cudaMemcpyAsync(grads, m->g, sizeof(float) * (size_t)m->nparam, cudaMemcpyDeviceToHost, m->stream);
     if (e != cudaSuccess) return mfail(m, OD_ERR_CUDA, cudaGetErrorString(e));
-    double l = 0;
-    const int rc = read_status(m, &l);
-    if (loss) *loss = l / ((double)valid * kOut);
-    return rc;
+    return read_status(m, loss, (double)valid * kOut);
 }
 
 // One Adam step on a batch gathered from device pools: features Xpool
@@ -1042,10 +1040,7 @@ int od_mlp_train_step(od_mlp* m, const void* Xpool, const void* Tpool, const lon
         e = od::launch_dependent(true, adam_kernel, tiles + 4, 256, 0, m->stream, A, tiles);
     }
     if (e != cudaSuccess) return mfail(m, OD_ERR_CUDA, cudaGetErrorString(e));
-    double l = 0;
-    const int rc = read_status(m, &l);
-    if (loss) *loss = l / ((double)batch * kOut);
-    return rc;
+    return read_status(m, loss, (double)batch * kOut);
 }
 
 // Normalisation of the closure's inputs and outputs.
