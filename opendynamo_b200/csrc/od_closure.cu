@@ -394,8 +394,8 @@ __global__ void apply_kernel(T* __restrict__ rhs, const float* __restrict__ Y, l
 // and transposed. Every kernel here that writes both goes through a tile of
 // 64 columns in shared memory and writes 16-byte chunks in both orientations
 // (a 2-byte store per value into the transposed copy touched a sector each:
-// at a batch of 8192 the gather took 80 us and the loss gradient 129 us, both
-// about 8 us of traffic).
+// at a batch of 8192 the gather took 81 us and the loss gradient 129 us, both
+// about 8 us of traffic; now 8 and 7).
 
 // shared-memory position of (row r, column c) of a tile of 64 columns: the
 // row's 16-byte chunks are XORed with its row group, so that whole-row writes
@@ -524,8 +524,9 @@ __global__ void __launch_bounds__(256) loss_grad_kernel(const float* Y, const fl
 
 // The end of the backward pass in one launch: bias gradients out[n] = sum_m
 // AT[n][m] (bf16 -> fp32) from the transposed copies, and the sums of the
-// weight gradients' K ranges. Launched one by one they took 35 and 27 us at a
-// batch of 8192, each waiting for its first loads alone; together 19 us.
+// weight gradients' K ranges. Launched one by one they took 69 and 28 us at a
+// batch of 8192 (2-byte loads, each waiting for its first ones alone); together
+// 19 us.
 //
 // Row sums, a warp per row: the order is that of 256 partial sums s[t] =
 // AT[n][t] + AT[n][t + 256] + ..., each 32 of them summed in a tree (t + 16,
@@ -627,7 +628,7 @@ constexpr int kAdamRows = 32;   // rows of a weight tile (of 64 columns)
 // weight tiles of 32 rows x 64 columns, which also write the bf16 copies W and
 // W^T and the fused inference kernel's weight image; the last four blocks: the
 // layers' biases. (Eight launches of one value a thread with 2-byte stores
-// into W^T, and a ninth for the image, took 39 us; this one 9 us.)
+// into W^T, and a ninth for the image, took 36 us; this one 9 us.)
 __global__ void __launch_bounds__(256) adam_kernel(const AdamArgs A, int tiles) {
     od::dependent_start();
     __shared__ __align__(16) bf16 tile[kAdamRows * 64];

@@ -1,6 +1,6 @@
-// Closure network kernels: the tcgen05 GEMM launcher and the small
-// element-wise kernels of MLP training (bf16 conversion, transposes, the
-// loss gradient, bias gradients, Adam).
+// Closure network: launches of the tcgen05 GEMM (one product, the grouped weight
+// gradients, the sums over K ranges), of the fused inference kernel and of its
+// weight image; self-tests.
 
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
@@ -82,9 +82,9 @@ __global__ void __launch_bounds__(kGemmThreads, 2) gemm_group_kernel(const GemmG
 // n <= kGroupMax fp32 products (no bias) in one launch, each split over K as
 // launch_gemm splits it; ksplit of each is set, and where it is above 1 its
 // partial sums are left in the product's own part of ws (the caller adds
-// them up). The weight gradients of the closure: four products of 3 to 28
-// tiles, 51 us launched one by one at a batch of 8192 (11 to 17 each), 40
-// together.
+// them up). The weight gradients of the closure: four products of 8 to 28
+// tiles, at a batch of 8192 89 us launched one by one before the swizzled
+// layout (16 to 39 each), 41 together.
 cudaError_t launch_gemm_group(GemmArgs* g, int n, float* ws, size_t ws_floats, cudaStream_t s) {
     if (n < 1 || n > kGroupMax) return cudaErrorInvalidValue;
     GemmGroup q{};
@@ -117,9 +117,12 @@ cudaError_t launch_gemm_group(GemmArgs* g, int n, float* ws, size_t ws_floats, c
 }
 
 // C = A B^T with the epilogue `epi`; M % 128 == 0, N % 64 == 0, K % 64 == 0.
-// Tile width: the widest of 256 / 128 / 64 dividing N that still gives two
-// CTAs per SM (the epilogue has four warps per CTA and wants company),
-// else 64. kStoreF32 products with few tiles and a long K (weight gradients)
+// Tile width: the widest of 256 / 128 / 64 dividing N of which there are two
+// tiles per SM, else 64 (fewer and wider tiles load A less often, but leave SMs
+// idle; tiles of 64 and 128 run two per SM, of 256 one). Forward pass, tiles of 64
+// / of 128 / by this rule: 8192 rows 57 / 75 / 57 us, 19072 rows 107 / 94 / 94,
+// 65536 rows 257 / 206 / 206 (just past two tiles of 256 per SM, at 38016 rows,
+// 128 would be better: 144 against 155). kStoreF32 products with few tiles and a long K (weight gradients)
 // split K when the caller passes a workspace of ksplit * M * N floats.
 cudaError_t launch_gemm(const GemmArgs& g0, int epi, cudaStream_t s, size_t ws_floats) {
     if (g0.M <= 0 || g0.N <= 0 || g0.K <= 0 || g0.M % BM || g0.N % 64 || g0.K % BK) return cudaErrorInvalidValue;

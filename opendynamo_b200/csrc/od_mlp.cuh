@@ -7,7 +7,6 @@
 // over all of K or over one of `ksplit` K ranges (blockIdx.z; fp32 partial
 // tiles, summed by a second kernel):
 //   - all threads stage 128 x 64 (A) and NT x 64 (B) bf16 blocks into shared
-//   - all threads stage 128 x 64 (A) and NT x 64 (B) bf16 blocks into shared
 //     memory with 16-byte cp.async copies, four stages deep for NT = 64 and
 //     three for the wider tiles, in the K-major 128-byte-swizzled layout of
 //     the tensor cores;
@@ -275,8 +274,8 @@ __device__ __forceinline__ void load_stage(const LoadPos& p, Smem<NT>& s, int st
 // of tensor and memory work): 256 threads, so that the epilogue's values are
 // spread over eight warps, two CTAs per SM. Forward products of a training
 // step (8192 x 256, K = 896 or 256, GELU epilogue), mean of the three layers,
-// cold caches: 26.0 us with 2-byte stores and eight lines per load phase,
-// 22.2 with 16-byte epilogue accesses, 11.8 with the swizzled layout too.
+// cold caches: 25.8 us with 128 threads, 2-byte stores and eight lines per load
+// phase, 11.9 with 256, 16-byte epilogue accesses and the swizzled layout.
 constexpr int kGemmThreads = 256;
 
 // One tile of one product: row block bx, column block by, K range bz. Called
