@@ -22,6 +22,10 @@ def _cuda_available():
 
 
 def pytest_collection_modifyitems(config, items):
+    # comparisons with the reference's own kernels need them built from its
+    # sources (oracle/build_ref.py), which not every machine has: run them last,
+    # so that a run that stops at its first failure has shown all the others
+    items.sort(key=lambda item: "test_gpu_reference" in item.nodeid)
     if _cuda_available():
         return
     skip = pytest.mark.skip(reason="no CUDA device")
